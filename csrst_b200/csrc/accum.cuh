@@ -30,7 +30,7 @@ namespace csrst {
 // lanes of the warp together; add() may be called by any subset.
 template <int TW, int TH, int OX, int OY>
 struct TileAcc {
-  static constexpr int kSize = TW * TH;
+  static constexpr int kSize = TW * TH, kTW = TW, kTH = TH, kOX = OX, kOY = OY;
   unsigned long long *tile;  // shared memory, kSize * stride entries, zeroed
   int stride;                // threads per CTA
   int bi, bj;                // warp-uniform base cell (window cells)

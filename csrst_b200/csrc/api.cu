@@ -482,8 +482,9 @@ int push_async(csrst_handle *h, int jcomp) {
       h->prepped = false;
     }
     if (!h->prepped) launch_prep32(h->ws, h->order, h->s);
-    launch_push32(push_args32(h, jcomp), h->order, h->s);
-    launch_after32(h->ws, h->prep_after ? 1 : 0, h->s);
+    Push32Args pa = push_args32(h, jcomp);
+    pa.prep_next = h->prep_after ? 1 : 0;
+    launch_push32(pa, h->order, h->s);
     h->prepped = h->prep_after;
     h->prep_after = false;
     h->pending = false;
@@ -787,8 +788,9 @@ int csrst_create(const csrst_config *cfg, csrst_handle **out) {
     }
   }
   if ((e = cudaMalloc(&h->mask, (size_t)Nx * Ny)) != cudaSuccess) return bad(e, "mask");
-  if ((e = cudaMalloc(&h->ws, sizeof(WinState))) != cudaSuccess) return bad(e, "window state");
-  if ((e = cudaMemsetAsync(h->ws, 0, sizeof(WinState), h->s)) != cudaSuccess) return bad(e, "memset");
+  const size_t wsb = sizeof(WinState) + sizeof(PushCtl);
+  if ((e = cudaMalloc(&h->ws, wsb)) != cudaSuccess) return bad(e, "window state");
+  if ((e = cudaMemsetAsync(h->ws, 0, wsb, h->s)) != cudaSuccess) return bad(e, "memset");
   const size_t nd = moments_scratch_doubles();
   if ((e = cudaMalloc(&h->dscratch, nd * sizeof(double))) != cudaSuccess) return bad(e, "diag");
   if ((e = cudaMalloc(&h->dmean, 8 * sizeof(double))) != cudaSuccess) return bad(e, "diag");

@@ -46,6 +46,7 @@ struct PushShared {
   double sb[4][32];  // block_bbox
   int tb[4];         // touched box of the CTA (window cells)
   int err;           // the member's sticky error at entry
+  bool last;         // this CTA ends its push last
 };
 
 __device__ __forceinline__ void bbox_reset(long long *b) {

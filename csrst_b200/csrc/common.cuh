@@ -61,6 +61,15 @@ struct WinState {
   int moves[2];               // last window move (moveI, moveJ)
 };
 
+// Launch bookkeeping of a member's pushes, in device memory right behind its
+// WinState (which checkpoints hold byte for byte).  Zero between launches but
+// for nofit.
+struct PushCtl {
+  unsigned done;  // CTAs that ended
+  int nofit;      // the next push's bunch does not fit the window (it reports the error)
+};
+__host__ __device__ inline PushCtl *push_ctl(WinState *ws) { return reinterpret_cast<PushCtl *>(ws + 1); }
+
 // One conformal cut cell (BoundaryCell, src/BoundaryCell.hh:28-47) after
 // SCBoundaryCondition::limitArea.
 struct CutCellDev {

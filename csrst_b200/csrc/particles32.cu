@@ -25,6 +25,7 @@
 #include "bunch32.cuh"
 #include "flux32.cuh"
 #include "kernels.cuh"
+#include "pushwork.cuh"
 #include "shapes.cuh"
 
 namespace csrst {
@@ -32,15 +33,71 @@ namespace {
 
 __device__ __forceinline__ long long gtid() { return blockIdx.x * (long long)blockDim.x + threadIdx.x; }
 
-struct View32 {
-  const float *base;  // window element of the particle's cell
-  int pitch;
-  __device__ __forceinline__ float operator()(int i, int j) const { return __ldg(base + (ptrdiff_t)j * pitch + i); }
+// 1D gather weights and first tap for an offset g in [0, 1) in a cell: along
+// an axis on which the component sits on the vertices (VERTEX) or half a cell
+// off them.  The taps are first, first + 1, ... relative to the cell; the
+// expressions are those of gather_edge / gather_cell (shapes.cuh).
+template <int ORDER>
+struct Taps32 {
+  static constexpr int N = ORDER + 2;
+  int first;
+  float w[N];
 };
-struct SumView32 {
-  View32 a, b;
-  __device__ __forceinline__ float operator()(int i, int j) const { return a(i, j) + b(i, j); }
-};
+template <int ORDER, bool VERTEX>
+__device__ __forceinline__ Taps32<ORDER> taps32(float g) {
+  Taps32<ORDER> t;
+  float d;
+  // with g in [0, 1) the floors of the general gather are 0 / 1 compares
+  if (VERTEX == (ORDER == 1)) {
+    // nearest point of the two around the offset: vertices for the quadratic
+    // shape, cell centres for the others
+    const bool up = g + 0.5f >= 1.0f;
+    const float l = ORDER == 1 ? (up ? 1.0f : 0.0f) : (up ? 0.5f : -0.5f);
+    d = g - l;
+    t.first = (up ? 1 : 0) - 1;
+  } else {
+    d = ORDER == 1 ? g - 0.5f : g;
+    t.first = ORDER == 1 ? -1 : 0;
+  }
+  if (ORDER == 0) {
+    t.w[0] = 1.0f - d; t.w[1] = d;
+  } else if (ORDER == 1) {
+    t.w[1] = 0.75f - d * d;
+    t.w[2] = 0.5f * (0.5f + d) * (0.5f + d);
+    t.w[0] = 1.0f - (t.w[1] + t.w[2]);
+  } else {
+    const float q = d * d;
+    t.w[1] = (float)(2.0 / 3.0) - q * (1.0f - 0.5f * d);
+    t.w[2] = (float)(2.0 / 3.0) - 0.5f * (1.0f - d) * (1.0f - q);
+    t.w[3] = (float)(1.0 / 6.0) * q * d;
+    t.w[0] = 1.0f - (t.w[1] + t.w[2] + t.w[3]);
+    t.first -= 1;
+  }
+  return t;
+}
+
+// One component at the taps: p is the plane's element of the particle's cell.
+// The cubic shape's last tap reads one column to the left, as the reference
+// does (ScatterGatherImpl.hh:467).
+template <int ORDER, bool SUM>
+__device__ __forceinline__ float gather32(const float *p, const float *p2, int pitch, const Taps32<ORDER> &x,
+                                          const Taps32<ORDER> &y) {
+  constexpr int N = Taps32<ORDER>::N;
+  const int o = y.first * pitch + x.first;
+  float r = 0.0f;
+#pragma unroll
+  for (int b = 0; b < N; ++b) {
+    float s = 0.0f;
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
+      const int k = o + b * pitch + (ORDER == 2 && a == N - 1 && b == N - 1 ? a - 1 : a);
+      const float f = SUM ? __ldg(p + k) + __ldg(p2 + k) : __ldg(p + k);
+      s = a == 0 ? x.w[0] * f : s + x.w[a] * f;
+    }
+    r = b == 0 ? y.w[0] * s : r + y.w[b] * s;
+  }
+  return r;
+}
 
 // Cell of the cell-relative coordinate t of cell c, as c' + 0.5 (exact).
 __device__ __forceinline__ double cellc(int c, float t) { return (double)(c + (int)floorf(t)) + 0.5; }
@@ -103,19 +160,23 @@ __device__ __forceinline__ void move32(const Push32Args &a, long long n, const I
   }
   const int wi = ci - WP0, wj = cj - WP1;
   // gather (FieldPatch::gather x3) anchored at the window cell of R1
-  const float c0 = floorf(x0), c1 = floorf(x1);
+  float c0 = floorf(x0), c1 = floorf(x1);
+  float g0 = x0 - c0, g1 = x1 - c1;
+  if (g0 >= 1.0f) { g0 = 0.0f; c0 += 1.0f; }  // a tiny negative coordinate rounded up to the next cell
+  if (g1 >= 1.0f) { g1 = 0.0f; c1 += 1.0f; }
   const int ai = wi + (int)c0, aj = wj + (int)c1;
   if (ai - 2 < -1 || ai + 2 > L0 || aj - 2 < -1 || aj + 2 > L1) {  // stencil outside the window planes
     set_err(ws, kErrWindowFit);
     m.ok = false;
     return;
   }
-  const float g0 = x0 - c0, g1 = x1 - c1;
-  const size_t o = (size_t)(aj + 1) * wp + (ai + 1);
-  const View32 vex{a.mEx + o, wp}, vey{a.mEy + o, wp}, vhx{a.mHx + o, wp}, vhy{a.mHy + o, wp};
-  const float E0 = gather_edge<ORDER_OF_PUSH>(vex, g0, g1, 0);
-  const float E1 = gather_edge<ORDER_OF_PUSH>(vey, g0, g1, 1);
-  const float Hf = gather_cell<ORDER_OF_PUSH>(SumView32{vhx, vhy}, g0, g1);
+  const int o = (aj + 1) * wp + (ai + 1);
+  // Ex sits half a cell off the vertices along x, Ey along y, Hz along both
+  const Taps32<ORDER_OF_PUSH> xv = taps32<ORDER_OF_PUSH, true>(g0), xc = taps32<ORDER_OF_PUSH, false>(g0);
+  const Taps32<ORDER_OF_PUSH> yv = taps32<ORDER_OF_PUSH, true>(g1), yc = taps32<ORDER_OF_PUSH, false>(g1);
+  const float E0 = gather32<ORDER_OF_PUSH, false>(a.mEx + o, nullptr, wp, xc, yv);
+  const float E1 = gather32<ORDER_OF_PUSH, false>(a.mEy + o, nullptr, wp, xv, yc);
+  const float Hf = gather32<ORDER_OF_PUSH, true>(a.mHx + o, a.mHy + o, wp, xc, yc);
   // hard-edge dipole at the absolute position of R1 (bend frame, FP64)
   const double X = a.org0 + ((double)ci + (double)x0) * a.h0, Y = a.org1 + ((double)cj + (double)x1) * a.h1;
   const double dist = a.chh * (X - a.Lb) - a.shh * (Y - a.hw);
@@ -161,62 +222,101 @@ struct Boxes32 {
   }
 };
 
-// The member's sticky error at entry, read by one thread for the CTA; a CTA
-// that sees one leaves as a whole.
-__device__ __forceinline__ bool entry_error(WinState *ws, PushShared &sh) {
-  if (threadIdx.x == 0) sh.err = *(volatile int *)&ws->err;
-  __syncthreads();
-  return sh.err != 0;
-}
+// Adds one particle's deposit to its warp's tile.  The whole stencil box is
+// checked against the tile once; inside it every entry is a load, an add and a
+// store at a compile-time offset from one address.  Boxes that do not fit go to
+// the tile or the window accumulator entry by entry.
+template <class Tile>
+struct TileSink {
+  unsigned long long *tile;  // this lane's tile
+  int bi, bj;                // its first window cell
+  int wi, wj;                // the particle's old cell (window cells)
+  unsigned long long *acc;
+  int L0, L1;
+  unsigned long long *p;
+  int j0;
+  bool in;
+  __device__ __forceinline__ TileSink(const Tile &t, int wi_, int wj_, unsigned long long *acc_, int L0_, int L1_)
+      : tile(t.tile), bi(t.bi - Tile::kOX), bj(t.bj - Tile::kOY), wi(wi_), wj(wj_), acc(acc_), L0(L0_), L1(L1_) {}
+  template <int NX, int NY>
+  __device__ __forceinline__ void box(int i, int j) {
+    const int a = wi + i - bi, b = wj + j - bj;
+    // a box larger than the tile (the cubic shape's general form) never fits
+    in = NX <= Tile::kTW && NY <= Tile::kTH && a >= 0 && a <= Tile::kTW - NX && b >= 0 && b <= Tile::kTH - NY;
+    p = tile + (b * Tile::kTW + a) * kPushThreads;
+    j0 = j;
+  }
+  template <int N>
+  __device__ __forceinline__ void row(int i, int j, const long long (&v)[N]) {
+    if (in) {
+#pragma unroll
+      for (int c = 0; c < N; ++c) p[((j - j0) * Tile::kTW + c) * kPushThreads] += (unsigned long long)v[c];
+    } else {
+#pragma unroll
+      for (int c = 0; c < N; ++c)
+        if (v[c] != 0) put(tile, wi + i + c - bi, wj + j - bj, acc, wi + i + c, wj + j, L0, L1, v[c]);
+    }
+  }
+  // one entry at (a, b) of the tile, window cell (i, j)
+  static __device__ __forceinline__ void put(unsigned long long *tile, int a, int b, unsigned long long *acc, int i, int j,
+                                          int L0, int L1, long long v) {
+    if ((unsigned)a < (unsigned)Tile::kTW && (unsigned)b < (unsigned)Tile::kTH)
+      tile[(b * Tile::kTW + a) * kPushThreads] += (unsigned long long)v;
+    else if (i >= 0 && j >= 0 && i < L0 && j < L1)
+      atomicAdd(&acc[j * L0 + i], (unsigned long long)v);
+  }
+};
 
-// The fused push of one CTA's share [beg, end) of one member: every lane
-// moves its particle, then the warp deposits the moves' flux (flux32.cuh)
-// into per-lane shared-memory tiles around a base cell the warp shares,
-// which drain into the member's window accumulator in global memory.  Called
-// by all threads of the CTA; ends with a barrier, so a CTA may run it for
-// several members in turn.
-template <int ORDER, int COMP>
-__device__ __forceinline__ void push32_range(const Push32Args &a, long long beg, long long end, PushShared &sh,
-                                             unsigned long long *sm) {
+// The fused push of one CTA's share of one member: every lane moves its
+// particle, then the warp deposits the moves' flux (flux32.cuh) into per-lane
+// shared-memory tiles around a base cell the warp shares, which drain into the
+// member's window accumulator in global memory.  Called by all threads of the
+// CTA; ends with a barrier, so a CTA may run it for several members in turn.
+template <int ORDER, int COMP, class Work>
+__device__ __forceinline__ void push32_range(const Push32Args &a, const Work &work, PushShared &sh, unsigned long long *sm) {
   if (entry_error(a.ws, sh)) return;  // the whole CTA leaves together
   WinState *ws = a.ws;
   const int L0 = ws->L0, L1 = ws->L1, WP0 = ws->P0, WP1 = ws->P1;
   using Tile = typename TileFor<ORDER>::T;
-  for (int k = threadIdx.x; k < Tile::kSize * (int)blockDim.x; k += blockDim.x) sm[k] = 0ull;
+  for (int k = threadIdx.x; k < Tile::kSize * kPushThreads; k += kPushThreads) sm[k] = 0ull;
   __syncthreads();
   Tile tile;
   tile.init(sm, L0, L1);
   Boxes32 box;
   bool overflow = false;
-  const long long rounds = end > beg ? (end - beg + blockDim.x - 1) / blockDim.x : 0;
-  // each lane's next particle is read while the current one moves
-  In32 next{};
-  if (beg + threadIdx.x < end) next = load32(a.b, beg + threadIdx.x);
-  for (long long it = 0; it < rounds; ++it) {  // the same rounds for every lane of the warp
-    const long long n = beg + it * blockDim.x + threadIdx.x;
-    const In32 cur = next;
-    if (n + blockDim.x < end) next = load32(a.b, n + blockDim.x);
-    Move32 m;
-    m.ok = false;
-    m.ci = WP0; m.cj = WP1;
-    if (n < end) {
-      move32<ORDER>(a, n, cur, L0, L1, WP0, WP1, m);
-      if (m.ok) box.add(m);
-    }
-    const int wi = m.ci - WP0, wj = m.cj - WP1;
-    tile.template rebase<false>(m.ok, wi, wj, a.acc, L0, L1);
-    // the compact form when every particle of the warp keeps its y base index
-    // and advances by at most one x base index
-    const int dx = m.ni - m.ci + base_index<ORDER>(m.o0) - base_index<ORDER>(m.a0);
-    const bool fast = !m.ok || ((unsigned)dx <= 1u && m.nj - m.cj + base_index<ORDER>(m.o1) == base_index<ORDER>(m.a1));
-    const bool all_fast = __all_sync(0xffffffffu, fast);
-    if (m.ok) {
+  long long n0, end, step;
+  for (int k = 0; work.run(k, n0, end, step); ++k) {
+    // each lane's next particle is read while the current one moves
+    In32 next{};
+    if (n0 + threadIdx.x < end) next = load32(a.b, n0 + threadIdx.x);
+    for (; n0 < end; n0 += step) {  // the same rounds for every lane of the warp
+      const long long n = n0 + threadIdx.x;
+      const In32 cur = next;
+      if (n + step < end) next = load32(a.b, n + step);
+      Move32 m;
+      m.ok = false;
+      m.ci = WP0; m.cj = WP1;
+      if (n < end) {
+        move32<ORDER>(a, n, cur, L0, L1, WP0, WP1, m);
+        if (m.ok) box.add(m);
+      }
+      const int wi = m.ci - WP0, wj = m.cj - WP1;
+      tile.template rebase<false>(m.ok, wi, wj, a.acc, L0, L1);
+      // the compact form when every particle of the warp keeps its y base index
+      // and advances by at most one x base index
+      const int dx = m.ni - m.ci + base_index<ORDER>(m.o0) - base_index<ORDER>(m.a0);
       const double K = (double)m.q * a.acc_scale;
-      auto sink = [&](int i, int j, long long v) { tile.template add<false>(wi + i, wj + j, v, a.acc, L0, L1); };
-      const bool ok = all_fast
-          ? flux_particle<ORDER, COMP, true>(m.a0, m.a1, m.ni - m.ci, m.nj - m.cj, m.o0, m.o1, K, __double2ll_rn(K), sink)
-          : flux_particle<ORDER, COMP, false>(m.a0, m.a1, m.ni - m.ci, m.nj - m.cj, m.o0, m.o1, K, __double2ll_rn(K), sink);
-      if (!ok) overflow = true;
+      const bool fast = !m.ok || ((unsigned)dx <= 1u && fabs(K) < kRoundMax &&
+                                  m.nj - m.cj + base_index<ORDER>(m.o1) == base_index<ORDER>(m.a1));
+      const bool all_fast = __all_sync(0xffffffffu, fast);
+      if (m.ok) {
+        TileSink<Tile> sink(tile, wi, wj, a.acc, L0, L1);
+        if (all_fast)
+          flux_compact<ORDER, COMP>(m.a0, m.a1, m.ni - m.ci, m.nj - m.cj, m.o0, m.o1, K, sink);
+        else if (!flux_particle<ORDER, COMP, false>(m.a0, m.a1, m.ni - m.ci, m.nj - m.cj, m.o0, m.o1, K,
+                                                    __double2ll_rn(K), sink))
+          overflow = true;
+      }
     }
   }
   tile.template flush<false>(a.acc, L0, L1);
@@ -225,18 +325,54 @@ __device__ __forceinline__ void push32_range(const Push32Args &a, long long beg,
   __syncthreads();
 }
 
+// Gather-patch set-up and the window-fit check from the box of the next
+// push's gather positions (cells of the static mesh).  defer: a bunch that does
+// not fit is reported by the next push, not at once (PushCtl).
+__device__ __forceinline__ void prep32_body(WinState *ws, int reach, bool defer) {
+  const int c = ws->cur;
+  const double mn0 = ord_dbl(ws->bb[c][0]), mn1 = ord_dbl(ws->bb[c][1]);
+  const double mx0 = ord_dbl(ws->bb[c][2]), mx1 = ord_dbl(ws->bb[c][3]);
+  int nofit = 0;
+  if (mn0 <= mx0) {
+    const int lp[4] = {(int)floor(mn0) - ws->P0, (int)floor(mx0) - ws->P0, (int)floor(mn1) - ws->P1,
+                       (int)floor(mx1) - ws->P1};
+    for (int k = 0; k < 4; ++k) ws->lp[k] = lp[k];
+    // every gather tap lies within [lp - reach, lp + reach]
+    nofit = lp[0] - reach < -1 || lp[1] + reach > ws->L0 || lp[2] - reach < -1 || lp[3] + reach > ws->L1;
+    if (nofit && !defer) set_err(ws, kErrWindowFit);
+  }
+  push_ctl(ws)->nofit = defer ? nofit : 0;
+  bbox_reset(ws->bb[1 - c]);
+  bbox_reset(ws->bball);
+}
+
+// Deposit bounds in window cells (PartBunch::getLocalPDomainInclOld).
+__device__ __forceinline__ void bounds32_body(WinState *ws) {
+  const double mn0 = ord_dbl(ws->bball[0]), mn1 = ord_dbl(ws->bball[1]);
+  const double mx0 = ord_dbl(ws->bball[2]), mx1 = ord_dbl(ws->bball[3]);
+  if (!(mn0 <= mx0)) { ws->gb[0] = 0; ws->gb[1] = -1; ws->gb[2] = 0; ws->gb[3] = -1; return; }
+  ws->gb[0] = (int)floor(mn0) - ws->P0; ws->gb[1] = (int)floor(mx0) - ws->P0;
+  ws->gb[2] = (int)floor(mn1) - ws->P1; ws->gb[3] = (int)floor(mx1) - ws->P1;
+}
+
 // CTAs per SM of the push launches: three for CIC and TSC, two for the
 // cubic shape, whose 5 x 5 stencil box needs more registers.
 template <int ORDER>
 struct Push32Occ { static constexpr int kCtas = ORDER == 2 ? 2 : 3; };
 
 template <int ORDER, int COMP>
-__global__ void __launch_bounds__(256, Push32Occ<ORDER>::kCtas) k_push32(Push32Args a) {
+__global__ void __launch_bounds__(kPushThreads, Push32Occ<ORDER>::kCtas) k_push32(Push32Args a) {
   extern __shared__ unsigned long long sacc[];
   __shared__ PushShared sh;
-  const long long per = (a.b.n + gridDim.x - 1) / gridDim.x;
-  const long long beg = (long long)blockIdx.x * per;
-  push32_range<ORDER, COMP>(a, beg, beg + per < a.b.n ? beg + per : a.b.n, sh, sacc);
+  push32_range<ORDER, COMP>(a, BunchWork{a.b.n}, sh, sacc);
+  // the last CTA swaps the box sets (the push filled the other one), derives
+  // the deposit bounds and, when nothing moves the particles or the window
+  // before the next push, sets up its gather patch
+  if (last_cta(a.ws, sh) && threadIdx.x == 0) {
+    a.ws->cur = 1 - a.ws->cur;
+    bounds32_body(a.ws);
+    if (a.prep_next) prep32_body(a.ws, 2, true);
+  }
 }
 
 // One push over a batch of FP32-mode members: the members' particles form one
@@ -244,7 +380,7 @@ __global__ void __launch_bounds__(256, Push32Occ<ORDER>::kCtas) k_push32(Push32A
 // equal contiguous shares, one per CTA; a CTA runs the push of every member
 // its share overlaps.
 template <int ORDER, int COMP>
-__global__ void __launch_bounds__(256, Push32Occ<ORDER>::kCtas) k_push32_batch(const Push32Args *args, const long long *ppre, int m,
+__global__ void __launch_bounds__(kPushThreads, Push32Occ<ORDER>::kCtas) k_push32_batch(const Push32Args *args, const long long *ppre, int m,
                                                        long long per) {
   extern __shared__ unsigned long long sacc[];
   __shared__ PushShared sh;
@@ -259,7 +395,7 @@ __global__ void __launch_bounds__(256, Push32Occ<ORDER>::kCtas) k_push32_batch(c
     __syncthreads();
     if (threadIdx.x == 0) sa = args[mm];
     __syncthreads();
-    push32_range<ORDER, COMP>(sa, lb, le, sh, sacc);
+    push32_range<ORDER, COMP>(sa, ShareWork{lb, le}, sh, sacc);
   }
 }
 
@@ -305,41 +441,13 @@ __global__ void k_flux32(const int *cell0, const float *a0, const float *a1, con
   }
 }
 
-// Gather-patch set-up and the window-fit check from the box of the next
-// push's gather positions (cells of the static mesh).
-__device__ __forceinline__ void prep32_body(WinState *ws, int reach) {
-  const int c = ws->cur;
-  const double mn0 = ord_dbl(ws->bb[c][0]), mn1 = ord_dbl(ws->bb[c][1]);
-  const double mx0 = ord_dbl(ws->bb[c][2]), mx1 = ord_dbl(ws->bb[c][3]);
-  if (mn0 <= mx0) {
-    const int lp[4] = {(int)floor(mn0) - ws->P0, (int)floor(mx0) - ws->P0, (int)floor(mn1) - ws->P1,
-                       (int)floor(mx1) - ws->P1};
-    for (int k = 0; k < 4; ++k) ws->lp[k] = lp[k];
-    // every gather tap lies within [lp - reach, lp + reach]
-    if (lp[0] - reach < -1 || lp[1] + reach > ws->L0 || lp[2] - reach < -1 || lp[3] + reach > ws->L1)
-      set_err(ws, kErrWindowFit);
-  }
-  bbox_reset(ws->bb[1 - c]);
-  bbox_reset(ws->bball);
-}
-
 __global__ void k_prep32(WinState *ws, int reach) {
-  if (threadIdx.x == 0) prep32_body(ws, reach);
+  if (threadIdx.x == 0) prep32_body(ws, reach, false);
 }
-
-// Deposit bounds in window cells (PartBunch::getLocalPDomainInclOld).
-__device__ __forceinline__ void bounds32_body(WinState *ws) {
-  const double mn0 = ord_dbl(ws->bball[0]), mn1 = ord_dbl(ws->bball[1]);
-  const double mx0 = ord_dbl(ws->bball[2]), mx1 = ord_dbl(ws->bball[3]);
-  if (!(mn0 <= mx0)) { ws->gb[0] = 0; ws->gb[1] = -1; ws->gb[2] = 0; ws->gb[3] = -1; return; }
-  ws->gb[0] = (int)floor(mn0) - ws->P0; ws->gb[1] = (int)floor(mx0) - ws->P0;
-  ws->gb[2] = (int)floor(mn1) - ws->P1; ws->gb[3] = (int)floor(mx1) - ws->P1;
-}
-
 
 __global__ void k_prep32_batch(const PrepArgs *p, int m) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < m) prep32_body(p[k].ws, 2);
+  if (k < m) prep32_body(p[k].ws, 2, false);
 }
 __global__ void k_after32_batch(const PrepArgs *p, int m) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -347,17 +455,6 @@ __global__ void k_after32_batch(const PrepArgs *p, int m) {
     p[k].ws->cur = 1 - p[k].ws->cur;
     bounds32_body(p[k].ws);
   }
-}
-
-// After a push: the box sets swap (the push filled the other one), the
-// deposit bounds follow from the push's boxes, and, when the caller knows
-// the next push reads the same particles and window (prep_next), its gather
-// patch is set up here too, which saves that push its own set-up launch.
-__global__ void k_after32(WinState *ws, int prep_next) {
-  if (threadIdx.x != 0) return;
-  ws->cur = 1 - ws->cur;
-  bounds32_body(ws);
-  if (prep_next) prep32_body(ws, 2);
 }
 
 __global__ void k_bbox32_clear(WinState *ws) {
@@ -491,7 +588,7 @@ int push_grid32() {
 
 template <int ORDER>
 void push32_order(const Push32Args &a, cudaStream_t s) {
-  const int g = push_grid32() / 3 * Push32Occ<ORDER>::kCtas;
+  const int g = push_ctas(a.b.n, push_grid32() / 3 * Push32Occ<ORDER>::kCtas);
   if (a.jcomp == 0) k_push32<ORDER, 0><<<g, 256, push_smem32<ORDER, 0>(), s>>>(a);
   else k_push32<ORDER, 1><<<g, 256, push_smem32<ORDER, 1>(), s>>>(a);
 }
@@ -558,8 +655,6 @@ void launch_prep32(WinState *ws, int order, cudaStream_t s) {
   (void)order;
   k_prep32<<<1, 32, 0, s>>>(ws, 2);
 }
-
-void launch_after32(WinState *ws, int prep_next, cudaStream_t s) { k_after32<<<1, 32, 0, s>>>(ws, prep_next); }
 
 void launch_bbox32(const Bunch32 &b, const Ref32 &R, int pending, WinState *ws, cudaStream_t s) {
   k_bbox32_clear<<<1, 32, 0, s>>>(ws);
