@@ -131,8 +131,8 @@ struct csrst_handle {
   double *ox = nullptr, *oy = nullptr;
   bool pending = false;
   bool fresh = false;  // loaded, no push yet
-  // FP32 mode: the last push's closing kernel set up the next push's gather
-  // patch (prepped); the next push is to do so (prep_after)
+  // the last push's last CTA set up the next push's gather patch (prepped);
+  // the next push is to do so (prep_after)
   bool prepped = false, prep_after = false;
   BBoxState bb = kBBInvalid;
   int push_grid = 0;
@@ -205,6 +205,7 @@ struct EnsPart {
   void *fey[2] = {nullptr, nullptr}, *fmv[2] = {nullptr, nullptr};
   int *tpre = nullptr, *bpre_ey = nullptr;
   int ney = 0;
+  size_t fix_smem = 0, tail_smem = 0;  // of the fix-up and step-tail launches (tail 0: a window is too large)
   unsigned *queue = nullptr;
 };
 
@@ -417,6 +418,7 @@ void free_particles(csrst_handle *h) {
   h->zfix = nullptr;
   drop_graphs(h);
   h->n = 0;
+  h->prepped = false;
 }
 
 int check_err(csrst_handle *h) {
@@ -447,7 +449,10 @@ PushArgs push_args(csrst_handle *h, int jcomp) {
   a.half = h->half;
   a.fact1 = h->half * h->cfg.charge_mass;
   a.fact2 = a.fact1 * kC;
-  a.h0 = h->b.hr0; a.h1 = h->b.hr1; a.dt = h->dt;
+  // a contribution is at most |q| c / (hx hy), and 4 n max|q| c / (hx hy) acc_scale <= 2^62
+  // (csrst_load_particles): below 2^51 for n >= 1024, with a factor of two to spare
+  a.narrow = h->n >= 1024 ? 1 : 0;
+  set_push_consts(a, h->order, h->b.hr0, h->b.hr1, h->dt);
   a.bz = h->cfg.bz; a.Lb = h->b.Lb; a.hw = 0.5 * h->b.w;
   a.chh = h->chh; a.shh = h->shh; a.bwidth = h->bwidth;
   return a;
@@ -473,18 +478,18 @@ Push32Args push_args32(csrst_handle *h, int jcomp) {
   return a;
 }
 
-// PartBunch::push_particles on the device (no host synchronisation).
-int push_async(csrst_handle *h, int jcomp) {
+// PartBunch::push_particles on the device, on stream s (no host synchronisation).
+int push_async(csrst_handle *h, int jcomp, cudaStream_t s) {
   const bool bb_ok = h->bb == kBBValid || (h->bb == kBBValidIfPending && h->pending);
   if (h->fp32) {
     if (!bb_ok) {
-      launch_bbox32(h->b32, h->R32, h->pending ? 1 : 0, h->ws, h->s);
+      launch_bbox32(h->b32, h->R32, h->pending ? 1 : 0, h->ws, s);
       h->prepped = false;
     }
-    if (!h->prepped) launch_prep32(h->ws, h->order, h->s);
+    if (!h->prepped) launch_prep32(h->ws, h->order, s);
     Push32Args pa = push_args32(h, jcomp);
     pa.prep_next = h->prep_after ? 1 : 0;
-    launch_push32(pa, h->order, h->s);
+    launch_push32(pa, h->order, s);
     h->prepped = h->prep_after;
     h->prep_after = false;
     h->pending = false;
@@ -494,13 +499,19 @@ int push_async(csrst_handle *h, int jcomp) {
     return CSRST_OK;
   }
   if (h->cfg.flags & CSRST_FLAG_KEEP_OLD) {  // keep oldR for inspection
-    k_set_pending_old<<<(unsigned)((h->n + 255) / 256), 256, 0, h->s>>>(h->x, h->y, h->px, h->py, h->n,
+    k_set_pending_old<<<(unsigned)((h->n + 255) / 256), 256, 0, s>>>(h->x, h->y, h->px, h->py, h->n,
                                                                        h->half, h->pending, h->ox, h->oy);
   }
-  if (!bb_ok) launch_bbox_next(h->x, h->y, h->px, h->py, h->n, h->half, h->pending, h->ws, h->s);
-  launch_push_prep(h->ws, h->b.hr0, h->b.hr1, h->order, h->s);
-  launch_push(push_args(h, jcomp), h->order, h->push_grid, h->s);
-  launch_global_bounds(h->ws, h->b.hr0, h->b.hr1, h->s);
+  if (!bb_ok) {
+    launch_bbox_next(h->x, h->y, h->px, h->py, h->n, h->half, h->pending, h->ws, s);
+    h->prepped = false;
+  }
+  if (!h->prepped) launch_push_prep(h->ws, h->b.hr0, h->b.hr1, h->order, s);
+  PushArgs pa = push_args(h, jcomp);
+  pa.prep_next = h->prep_after ? 1 : 0;
+  launch_push(pa, h->order, h->push_grid, s);
+  h->prepped = h->prep_after;
+  h->prep_after = false;
   h->pending = false;
   h->fresh = false;
   h->bb = kBBValidIfPending;
@@ -562,6 +573,7 @@ void update_e_async(csrst_handle *h, int comp) {
 }
 
 void move_async(csrst_handle *h) {
+  h->prepped = false;  // the set-up is relative to the window
   if (h->fp32) launch_move(field_args32(h, 0), h->scratchf, h->b.hr0, h->b.hr1, h->s);
   else launch_move(field_args(h, 0), h->scratch, h->b.hr0, h->b.hr1, h->s);
 }
@@ -640,11 +652,11 @@ int fused_fields_async(csrst_handle *h) {
     const PlaneT<float> dst[4] = {{h->ExfB, h->pitch32}, {h->EyfB, h->pitch32}, {h->HxfB, h->pitch32},
                                   {h->HyfB, h->pitch32}};
     rc = launch_yee_fused(field_args32(h, 0), dst, h->kind, h->kpitch, h->cutidx, static_cast<float *>(h->zfix),
-                          h->zpitch, h->zrows, g_staging_polls, h->s, h->s2, h->fork, h->join);
+                          h->zpitch, h->zrows, g_staging_polls, h->s, h->s2, h->fork);
   } else {
     const Plane dst[4] = {{h->ExB, h->pitch}, {h->EyB, h->pitch}, {h->HxB, h->pitch}, {h->HyB, h->pitch}};
     rc = launch_yee_fused(field_args(h, 0), dst, h->kind, h->kpitch, h->cutidx, static_cast<double *>(h->zfix),
-                          h->zpitch, h->zrows, g_staging_polls, h->s, h->s2, h->fork, h->join);
+                          h->zpitch, h->zrows, g_staging_polls, h->s, h->s2, h->fork);
   }
   if (rc != kOk) return fail(h, rc == kErrArg ? CSRST_E_ARG : CSRST_E_CUDA, "fused field sweep: tensor-map set-up");
   h->acc_fresh[0] = false;
@@ -659,9 +671,26 @@ void window_ey_async(csrst_handle *h) {
   h->acc_fresh[1] = false;
 }
 
-void mark(csrst_handle *h, int k) {
-  if (h->tev) cudaEventRecord(h->tev[k], h->s);
+bool tail_fits(const csrst_handle *h) {
+  return (h->fp32 ? step_tail_smem<float>(h->L0, h->L1) : step_tail_smem<double>(h->L0, h->L1)) > 0;
 }
+
+// The window's Ey, the trailing half drift (owed), the window move and the
+// next push's set-up in one launch; false if the window is too large for it.
+bool step_tail_async(csrst_handle *h) {
+  const int ran = h->fp32 ? launch_step_tail(field_args32(h, 1), h->b.hr0, h->b.hr1, h->order, h->s)
+                          : launch_step_tail(field_args(h, 1), h->b.hr0, h->b.hr1, h->order, h->s);
+  if (!ran) return false;
+  h->acc_fresh[1] = false;
+  drift_back(h);
+  h->prepped = true;
+  return true;
+}
+
+void mark_on(csrst_handle *h, int k, cudaStream_t s) {
+  if (h->tev) cudaEventRecord(h->tev[k], s);
+}
+void mark(csrst_handle *h, int k) { mark_on(h, k, h->s); }
 
 // TETMSolver::updateField_firstStep + updateField_secondStep + moveMesh.
 // Events 0..7 (csrst_step_timed) bracket the pushes, the field work of each
@@ -669,10 +698,9 @@ void mark(csrst_handle *h, int k) {
 int step_async(csrst_handle *h) {
   mark(h, 0);
   // in the fused step nothing moves the particles or the window between the
-  // two pushes: the first push's closing kernel also sets up the second
-  h->prepped = false;
-  h->prep_after = h->fp32 && fused_ok(h);
-  push_async(h, 0);
+  // two pushes: the first push's last CTA also sets up the second
+  h->prep_after = fused_ok(h);
+  push_async(h, 0, h->s);
   mark(h, 1);
   if (fused_ok(h)) {
     const int rc = fused_fields_async(h);
@@ -682,9 +710,19 @@ int step_async(csrst_handle *h) {
     }
     mark(h, 2);
     drift_back(h);
-    mark(h, 3);
-    push_async(h, 1);
-    mark(h, 4);
+    // the second push reads the window, which the fix-up alone writes: it
+    // follows the fix-up on s2 while the tiles run on
+    mark_on(h, 3, h->s2);
+    push_async(h, 1, h->s2);
+    mark_on(h, 4, h->s2);
+    cudaEventRecord(h->join, h->s2);
+    cudaStreamWaitEvent(h->s, h->join, 0);
+    if (step_tail_async(h)) {
+      mark(h, 5);
+      mark(h, 6);
+      mark(h, 7);
+      return CSRST_OK;
+    }
     window_ey_async(h);
   } else {
     half_h_async(h);
@@ -693,7 +731,7 @@ int step_async(csrst_handle *h) {
     mark(h, 2);
     drift_back(h);
     mark(h, 3);
-    push_async(h, 1);
+    push_async(h, 1, h->s);
     mark(h, 4);
     update_e_async(h, 1);
   }
@@ -812,7 +850,7 @@ int csrst_create(const csrst_config *cfg, csrst_handle **out) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  h->push_grid = 3 * sms;  // single-member FP64 push: three CTAs per SM
+  h->push_grid = kPushCtas * sms;  // single-member FP64 push
   *out = h;
   return CSRST_OK;
 }
@@ -1251,7 +1289,7 @@ int csrst_push(csrst_handle *h, int jcomp) {
   int rc = need_bunch(h);
   if (rc) return rc;
   if (jcomp != 0 && jcomp != 1) return fail(h, CSRST_E_ARG, "jcomp must be 0 or 1");
-  push_async(h, jcomp);
+  push_async(h, jcomp, h->s);
   return CSRST_OK;
 }
 
@@ -1293,7 +1331,7 @@ int csrst_move_window(csrst_handle *h) {
 int csrst_step_first(csrst_handle *h) {
   int rc = need_bunch(h);
   if (rc) return rc;
-  push_async(h, 0);
+  push_async(h, 0, h->s);
   half_h_async(h);
   update_e_async(h, 0);
   half_h_async(h);
@@ -1304,7 +1342,7 @@ int csrst_step_first(csrst_handle *h) {
 int csrst_step_second(csrst_handle *h) {
   int rc = need_bunch(h);
   if (rc) return rc;
-  push_async(h, 1);
+  push_async(h, 1, h->s);
   update_e_async(h, 1);
   drift_back(h);
   return CSRST_OK;
@@ -1315,14 +1353,15 @@ int csrst_step(csrst_handle *h, int nsteps) {
   if (rc) return rc;
   if (nsteps < 0) return fail(h, CSRST_E_ARG, "nsteps < 0");
   // The graph is recorded in the steady state of the loop: the stored
-  // positions owe the trailing -dt/2 drift and the box of the next gather
-  // positions is current.  Anything else runs one step eagerly first.
-  while (nsteps > 0 && !(h->pending && h->bb == kBBValid)) {
+  // positions owe the trailing -dt/2 drift, the box of the next gather
+  // positions is current, and the last step's end has set up the first push
+  // (where it does so).  Anything else runs one step eagerly first.
+  const bool fused = fused_ok(h), tail = fused && tail_fits(h);
+  while (nsteps > 0 && !(h->pending && h->bb == kBBValid && h->prepped == tail)) {
     if ((rc = step_async(h))) return rc;
     --nsteps;
   }
   if (nsteps == 0) return CSRST_OK;
-  const bool fused = fused_ok(h);
   if (fused != h->graph_fused) {
     drop_graphs(h);
     h->graph_fused = fused;
@@ -1339,7 +1378,7 @@ int csrst_step(csrst_handle *h, int nsteps) {
         return rc;
       }
       if (ce != cudaSuccess) return cuda_fail(h, ce, "cudaStreamEndCapture");
-      cudaError_t e = cudaGraphInstantiate(&h->graph[p], g, 0);
+      cudaError_t e = cudaGraphInstantiate(&h->graph[p], g, cudaGraphInstantiateFlagUseNodePriority);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return cuda_fail(h, e, "cudaGraphInstantiate");
     } else if (fused) {
@@ -1580,6 +1619,9 @@ cudaError_t part_build_fused_t(csrst_ensemble *e, EnsPart &P) {
       }
     }
     bey.push_back(bey.back() + (h->L0 * h->L1 + h->L1 + 2 + 255) / 256);
+    P.fix_smem = std::max(P.fix_smem, fixup_smem<T>(h->L0, h->L1));
+    const size_t tb = step_tail_smem<T>(h->L0, h->L1);
+    P.tail_smem = k > 0 && P.tail_smem == 0 ? 0 : tb == 0 ? 0 : std::max(P.tail_smem, tb);
   }
   for (int p = 0; p < 2; ++p) {
     P.ytile[p] = dev_copy(tile[p], err);
@@ -1757,8 +1799,11 @@ template <class T>
 void part_fields_fused(const csrst_ensemble *e, EnsPart &P, int half) {
   const int p = e->epar;
   if (half == 0) {  // the static sweep of the whole step and the window's half H, Ex, half H
-    launch_yee_batch<T>(P.ytile[p], P.yfix[p], P.tpre, P.m, P.queue, P.s);
-  } else {          // the window's Ey (after the second push), then the window move
+    launch_yee_batch<T>(P.ytile[p], P.yfix[p], P.tpre, P.m, P.fix_smem, P.queue, P.s, P.s2, P.fork, P.join);
+  } else if (P.tail_smem > 0) {  // the window's Ey (after the second push) and the window move
+    launch_step_tail_batch<T>(static_cast<const FieldArgsT<T> *>(P.fey[p]), static_cast<const MoveArgs<T> *>(P.fmv[p]),
+                              P.m, P.tail_smem, P.s);
+  } else {
     launch_window_ey_batch<T>(static_cast<const FieldArgsT<T> *>(P.fey[p]), P.bpre_ey, P.m, P.ney, P.s);
     launch_move_batch<T>(static_cast<const MoveArgs<T> *>(P.fmv[p]), P.m, P.s);
   }
@@ -1832,6 +1877,7 @@ void ensemble_mark(csrst_ensemble *e) {
     h->pending = true;
     h->bb = kBBValid;
     h->fresh = false;
+    h->prepped = false;  // the batch sets its pushes up itself
     h->acc_fresh[0] = h->acc_fresh[1] = false;
   }
 }

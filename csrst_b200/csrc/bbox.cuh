@@ -40,10 +40,41 @@ __device__ __forceinline__ void block_bbox(double mn0, double mn1, double mx0, d
   __syncthreads();
 }
 
+// Smallest ordered-integer double of a warp: its high words, then the low
+// words of the lanes that hold that high word.
+__device__ __forceinline__ long long warp_min_ord(long long v) {
+  const int hi = (int)(v >> 32), mh = __reduce_min_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)v : 0xffffffffu);
+  return ((long long)mh << 32) | ml;
+}
+
+// The boxes of one push, merged over a CTA into ws->bball (v[0 .. 3]: R0 u R2)
+// and the next push's slot (v[4 .. 7]), as ordered-integer doubles, the maxima
+// complemented (~x reverses the order), so that everything is a minimum; sb is
+// shared scratch.  Ends with a barrier.
+__device__ __forceinline__ void merge_boxes(const long long (&v)[8], WinState *ws, long long (*sb)[32]) {
+  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const long long m = warp_min_ord(v[k]);
+    if ((threadIdx.x & 31) == 0) sb[k][w] = m;
+  }
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    const int k = threadIdx.x;
+    long long m = sb[k][0];
+    for (int q = 1; q < nw; ++q) m = sb[k][q] < m ? sb[k][q] : m;
+    long long *dst = (k < 4 ? ws->bball : ws->bb[1 - ws->cur]) + (k & 3);
+    if ((k & 3) < 2) atomicMin(dst, m);
+    else atomicMax(dst, ~m);
+  }
+  __syncthreads();
+}
+
 // Shared scratch of one push CTA, declared once per kernel so that a kernel
 // that inlines several push variants does not hold one copy per variant.
 struct PushShared {
-  double sb[4][32];  // block_bbox
+  long long sb[8][32];  // merge_boxes
   int tb[4];         // touched box of the CTA (window cells)
   int err;           // the member's sticky error at entry
   bool last;         // this CTA ends its push last

@@ -65,8 +65,10 @@ struct WinState {
 // WinState (which checkpoints hold byte for byte).  Zero between launches but
 // for nofit.
 struct PushCtl {
+  unsigned next;  // runs of particles handed out
   unsigned done;  // CTAs that ended
   int nofit;      // the next push's bunch does not fit the window (it reports the error)
+  int pad;
 };
 __host__ __device__ inline PushCtl *push_ctl(WinState *ws) { return reinterpret_cast<PushCtl *>(ws + 1); }
 

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "pushwork.cuh"
 #include "tma.cuh"
 
 namespace csrst {
@@ -112,21 +113,19 @@ __device__ __forceinline__ void half_h_static(const FieldArgsT<T> &a, int b) {
   store_masked(hyp, hy, m);
 }
 
-// Window cell k (x fastest) of the half H sub-step.
+// Window cell (i, j) of the half H sub-step.
 template <class T>
-__device__ __forceinline__ void window_h(const FieldArgsT<T> &a, int k) {
-  const int i = k % a.L0, j = k / a.L0;
+__device__ __forceinline__ void window_h(const FieldArgsT<T> &a, int i, int j) {
   T &hx = a.mHx.at(i, j), &hy = a.mHy.at(i, j);
   hx = hx - a.chx * (a.mEy.at(i + 1, j) - a.mEy.at(i, j));
   hy = hy + a.chy * (a.mEx.at(i, j + 1) - a.mEx.at(i, j));
 }
 
-// Window cell k of the E sub-step: the window current comes from the
+// Window cell (i, j) = k (x fastest) of the E sub-step: the window current comes from the
 // fixed-point accumulator of the last push, which is converted, stored for
 // diagnostics and cleared for the next deposit.
 template <class T, int COMP>
-__device__ __forceinline__ void window_e(const FieldArgsT<T> &a, int k) {
-  const int i = k % a.L0, j = k / a.L0;
+__device__ __forceinline__ void window_e(const FieldArgsT<T> &a, int k, int i, int j) {
   const T J = (T)((double)(long long)a.acc[k] * a.acc_inv);
   a.acc[k] = 0ull;
   if (COMP == 0) {
@@ -171,7 +170,7 @@ __device__ __forceinline__ void half_h_body(const FieldArgsT<T> &a, int b) {
   } else {
     const int k = (b - a.nbS - a.nbC - a.nbP) * blockDim.x + threadIdx.x;
     if (k >= a.L0 * a.L1) return;
-    window_h(a, k);
+    window_h(a, k % a.L0, k / a.L0);
   }
 }
 
@@ -266,7 +265,7 @@ __device__ __forceinline__ void update_e_body(const FieldArgsT<T> &a, int b, T z
   } else {
     const int k = (b - a.nbS - a.nbC - a.nbP) * blockDim.x + threadIdx.x;
     if (k >= a.L0 * a.L1) return;
-    window_e<T, COMP>(a, k);
+    window_e<T, COMP>(a, k, k % a.L0, k / a.L0);
   }
 }
 
@@ -324,6 +323,23 @@ __device__ __forceinline__ void exchange_body(const FieldArgsT<T> &a, int which,
   }
 }
 
+// f(c, r) for the cells of a w x h rectangle over threads tid of nth.  ROWS: a
+// warp a row at a time, which needs no division per cell (one CTA: its time is
+// instructions); else one cell after another (a cluster: its time is latency,
+// and rows would leave most of its warps idle).
+template <bool ROWS, class F>
+__device__ __forceinline__ void for_cells(int w, int h, int tid, int nth, F &&f) {
+  if (ROWS) {
+    for (int r = tid >> 5; r < h; r += nth >> 5)
+      for (int c = threadIdx.x & 31; c < w; c += 32) f(c, r);
+  } else {
+    for (int k = tid; k < w * h; k += nth) {
+      const int r = k / w;
+      f(k - r * w, r);
+    }
+  }
+}
+
 // Copy the static fields into the window interior (Communicator::copy via
 // copyFields, main.cpp:335-337).
 template <class T>
@@ -341,8 +357,7 @@ __global__ void k_copy_to_window(FieldArgsT<T> a) {
 // regular inside cell: the fused sub-step launches assume the strip exchange
 // and the cut-cell (or absorbing-layer) updates never meet.
 template <class T>
-__device__ void check_window_clear(const FieldArgsT<T> &a, WinState *ws) {
-  const int P0 = ws->P0, P1 = ws->P1;
+__device__ void check_window_clear(const FieldArgsT<T> &a, int P0, int P1) {
   const int per = 2 * (a.L0 + 2) + 2 * a.L1;
   for (int k = threadIdx.x; k < per; k += blockDim.x) {
     int i, j;
@@ -353,12 +368,12 @@ __device__ void check_window_clear(const FieldArgsT<T> &a, WinState *ws) {
     const int si = i + P0, sj = j + P1;
     if (si < 0 || sj < 0 || si >= a.Nx || sj >= a.Ny || !a.mask[(size_t)sj * a.Nx + si] ||
         (a.pml_rows && (si < a.pml_rows[sj].x || si >= a.pml_rows[sj].y)))  // or an absorbing-layer cell
-      set_err(ws, kErrWindowWall);
+      set_err(a.ws, kErrWindowWall);
   }
 }
 
 template <class T>
-__global__ void k_check_window(FieldArgsT<T> a) { check_window_clear(a, a.ws); }
+__global__ void k_check_window(FieldArgsT<T> a) { check_window_clear(a, a.ws->P0, a.ws->P1); }
 
 // Window move (moveMesh, main.cpp:562-652, and exchangeBoundariesMovingMesh,
 // Communicator.cpp:123-642): from the last deposit's particle bounds the
@@ -446,81 +461,92 @@ __device__ __forceinline__ void move_body(const MoveArgs<T> &m) {
   move_finish(m, moveI, m1);
 }
 
-// Position, origin and strips after the shifted copy (one CTA).
+// The strip layers of a move: type 0..2 window -> static (Hz, Ex, Ey), 3..5
+// static -> window, each a rectangle of window (0..2) or static (3..5) cells,
+// with the first item of each; in the reference's list order (slot 2 t: the
+// move in x, 2 t + 1: in y).
+struct StripLayers {
+  int lay[12][4];  // x0, x1, y0, y1 (inclusive)
+  int beg[13];
+};
+
+// Fills the layers of a move to window position (P0, P1) (one CTA; P0, P1
+// after the move): 12 threads a layer each, one the prefix sum.
 template <class T>
-__device__ __forceinline__ void move_finish(const MoveArgs<T> &m, int moveI, int m1) {
-  const FieldArgsT<T> &a = m.f;
-  WinState *ws = a.ws;
-  if (threadIdx.x == 0) {
-    ws->P0 += moveI; ws->P1 += m1;
-    ws->mo0 += moveI * m.h0;
-    ws->mo1 += m1 * m.h1;
-  }
-  __syncthreads();
-  // phase C: strip layers; type 0..2 window -> static (Hz, Ex, Ey), 3..5 static -> window.
-  const int P0 = ws->P0, P1 = ws->P1, Ld0 = a.L0 - 1, Ld1 = a.L1 - 1;
-  int lay[12][5], nl = 0;
-  auto add = [&](int t, int b0, int e0, int b1, int e1) {
-    lay[nl][0] = t; lay[nl][1] = b0; lay[nl][2] = e0; lay[nl][3] = b1; lay[nl][4] = e1; ++nl;
-  };
-  // layers grouped by type, in the reference's list order
-  for (int t = 0; t < 6; ++t) {
-    if (moveI == 1) {
-      switch (t) {
-        case 0: add(0, -1, -1, -m1, Ld1 - m1 - 1); break;
-        case 1: add(1, -1, -1, 1 - m1, Ld1 - m1); break;
-        case 2: add(2, 0, 0, -m1, Ld1 - m1); break;
-        case 3: add(3, Ld0 + P0, Ld0 + P0, P1, Ld1 + P1); break;
-        case 4: add(4, Ld0 + P0, Ld0 + P0, P1, Ld1 + P1 + 1); break;
-        case 5: add(5, Ld0 + P0 + 1, Ld0 + P0 + 1, P1, Ld1 + P1); break;
+__device__ __forceinline__ void strip_layers(StripLayers &S, const FieldArgsT<T> &a, int moveI, int m1, int P0, int P1) {
+  if (threadIdx.x < 12) {
+    const int l = threadIdx.x, t = l >> 1, Ld0 = a.L0 - 1, Ld1 = a.L1 - 1;
+    int y[4] = {0, -1, 0, -1};
+    auto set = [&](int b0, int e0, int b1, int e1) { y[0] = b0; y[1] = e0; y[2] = b1; y[3] = e1; };
+    if ((l & 1) == 0) {
+      if (moveI == 1) {
+        switch (t) {
+          case 0: set(-1, -1, -m1, Ld1 - m1 - 1); break;
+          case 1: set(-1, -1, 1 - m1, Ld1 - m1); break;
+          case 2: set(0, 0, -m1, Ld1 - m1); break;
+          case 3: set(Ld0 + P0, Ld0 + P0, P1, Ld1 + P1); break;
+          case 4: set(Ld0 + P0, Ld0 + P0, P1, Ld1 + P1 + 1); break;
+          default: set(Ld0 + P0 + 1, Ld0 + P0 + 1, P1, Ld1 + P1); break;
+        }
       }
-    }
-    if (m1 == 1) {
+    } else if (m1 == 1) {
       switch (t) {
-        case 0: add(0, -moveI, Ld0 - 1 - moveI, -1, -1); break;
-        case 1: add(1, -moveI, Ld0 - moveI, 0, 0); break;
-        case 2: add(2, 1 - moveI, Ld0 - moveI, -1, -1); break;
-        case 3: add(3, P0, Ld0 + P0, Ld1 + P1, Ld1 + P1); break;
-        case 4: add(4, P0, Ld0 + P0, Ld1 + 1 + P1, Ld1 + 1 + P1); break;
-        case 5: add(5, P0, Ld0 + P0 + 1, Ld1 + P1, Ld1 + P1); break;
+        case 0: set(-moveI, Ld0 - 1 - moveI, -1, -1); break;
+        case 1: set(-moveI, Ld0 - moveI, 0, 0); break;
+        case 2: set(1 - moveI, Ld0 - moveI, -1, -1); break;
+        case 3: set(P0, Ld0 + P0, Ld1 + P1, Ld1 + P1); break;
+        case 4: set(P0, Ld0 + P0, Ld1 + 1 + P1, Ld1 + 1 + P1); break;
+        default: set(P0, Ld0 + P0 + 1, Ld1 + P1, Ld1 + P1); break;
       }
     } else if (m1 == -1) {
       switch (t) {
-        case 0: add(0, -moveI, Ld0 - moveI - 1, Ld1, Ld1); break;
-        case 1: add(1, -moveI, Ld0 - moveI, Ld1 + 1, Ld1 + 1); break;
-        case 2: add(2, 1 - moveI, Ld0 - moveI, Ld1 + 1, Ld1 + 1); break;
-        case 3: add(3, P0, Ld0 + P0, P1 - 1, P1 - 1); break;
-        case 4: add(4, P0, Ld0 + P0, P1, P1); break;
-        case 5: add(5, P0, Ld0 + P0 + 1, P1, P1); break;
+        case 0: set(-moveI, Ld0 - moveI - 1, Ld1, Ld1); break;
+        case 1: set(-moveI, Ld0 - moveI, Ld1 + 1, Ld1 + 1); break;
+        case 2: set(1 - moveI, Ld0 - moveI, Ld1 + 1, Ld1 + 1); break;
+        case 3: set(P0, Ld0 + P0, P1 - 1, P1 - 1); break;
+        case 4: set(P0, Ld0 + P0, P1, P1); break;
+        default: set(P0, Ld0 + P0 + 1, P1, P1); break;
       }
     }
-  }
-  // clip each layer (window layers to [-1, L] and the static domain; static
-  // layers to the static domain and the window incl. guards)
-  int beg[13];
-  beg[0] = 0;
-  for (int l = 0; l < nl; ++l) {
-    int *y = lay[l];
-    if (y[0] < 3) {
-      y[1] = max(max(y[1], -1), -P0); y[2] = min(min(y[2], a.L0), a.Nx - 1 - P0);
-      y[3] = max(max(y[3], -1), -P1); y[4] = min(min(y[4], a.L1), a.Ny - 1 - P1);
+    // window layers clipped to [-1, L] and the static domain; static layers to
+    // the static domain and the window incl. guards
+    if (t < 3) {
+      y[0] = max(max(y[0], -1), -P0); y[1] = min(min(y[1], a.L0), a.Nx - 1 - P0);
+      y[2] = max(max(y[2], -1), -P1); y[3] = min(min(y[3], a.L1), a.Ny - 1 - P1);
     } else {
-      y[1] = max(max(y[1], 0), P0 - 1); y[2] = min(min(y[2], a.Nx - 1), P0 + a.L0);
-      y[3] = max(max(y[3], 0), P1 - 1); y[4] = min(min(y[4], a.Ny - 1), P1 + a.L1);
+      y[0] = max(max(y[0], 0), P0 - 1); y[1] = min(min(y[1], a.Nx - 1), P0 + a.L0);
+      y[2] = max(max(y[2], 0), P1 - 1); y[3] = min(min(y[3], a.Ny - 1), P1 + a.L1);
     }
-    const int c = (y[2] >= y[1] && y[4] >= y[3]) ? (y[2] - y[1] + 1) * (y[4] - y[3] + 1) : 0;
-    beg[l + 1] = beg[l] + c;
+    const bool any = ((l & 1) ? m1 != 0 : moveI == 1) && y[1] >= y[0] && y[3] >= y[2];
+    for (int q = 0; q < 4; ++q) S.lay[l][q] = y[q];
+    S.beg[l + 1] = any ? (y[1] - y[0] + 1) * (y[3] - y[2] + 1) : 0;
   }
-  const int total = beg[nl];
-  T *vals = m.scratch;  // the snapshot is no longer needed
-  for (int k = threadIdx.x; k < total; k += blockDim.x) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    S.beg[0] = 0;
+    for (int l = 0; l < 12; ++l) S.beg[l + 1] += S.beg[l];
+  }
+  __syncthreads();
+}
+
+// The strips of a move (one CTA): every value is read before any is written;
+// vals holds one per item.
+template <class T>
+__device__ __forceinline__ void move_strips(const FieldArgsT<T> &a, const StripLayers &S, int P0, int P1, T *vals) {
+  const int total = S.beg[12];
+  auto item = [&](int k, int &t, int &i, int &j) {
     int l = 0;
-    while (k >= beg[l + 1]) ++l;
-    const int *y = lay[l];
-    const int w = y[2] - y[1] + 1, r = k - beg[l];
-    const int i = y[1] + r % w, j = y[3] + r / w;
+    while (k >= S.beg[l + 1]) ++l;
+    const int w = S.lay[l][1] - S.lay[l][0] + 1, r = k - S.beg[l];
+    t = l >> 1;
+    i = S.lay[l][0] + r % w;
+    j = S.lay[l][2] + r / w;
+  };
+  for (int k = threadIdx.x; k < total; k += blockDim.x) {
+    int t, i, j;
+    item(k, t, i, j);
     T v;
-    switch (y[0]) {
+    switch (t) {
       case 0: v = a.mHx.at(i, j) + a.mHy.at(i, j); break;
       case 1: v = a.mEx.at(i, j); break;
       case 2: v = a.mEy.at(i, j); break;
@@ -532,13 +558,10 @@ __device__ __forceinline__ void move_finish(const MoveArgs<T> &m, int moveI, int
   }
   __syncthreads();
   for (int k = threadIdx.x; k < total; k += blockDim.x) {
-    int l = 0;
-    while (k >= beg[l + 1]) ++l;
-    const int *y = lay[l];
-    const int w = y[2] - y[1] + 1, r = k - beg[l];
-    const int i = y[1] + r % w, j = y[3] + r / w;
+    int t, i, j;
+    item(k, t, i, j);
     const T v = vals[k];
-    switch (y[0]) {
+    switch (t) {
       case 0: a.Hx.at(i + P0, j + P1) = T(0.5) * v; a.Hy.at(i + P0, j + P1) = T(0.5) * v; break;
       case 1: a.Ex.at(i + P0, j + P1) = v; break;
       case 2: a.Ey.at(i + P0, j + P1) = v; break;
@@ -547,8 +570,25 @@ __device__ __forceinline__ void move_finish(const MoveArgs<T> &m, int moveI, int
       default: a.mEy.at(i - P0, j - P1) = v; break;
     }
   }
+}
+
+// Position, origin and strips after the shifted copy (one CTA).
+template <class T>
+__device__ __forceinline__ void move_finish(const MoveArgs<T> &m, int moveI, int m1) {
+  const FieldArgsT<T> &a = m.f;
+  WinState *ws = a.ws;
+  __shared__ StripLayers S;
+  if (threadIdx.x == 0) {
+    ws->P0 += moveI; ws->P1 += m1;
+    ws->mo0 += moveI * m.h0;
+    ws->mo1 += m1 * m.h1;
+  }
   __syncthreads();
-  check_window_clear(a, ws);
+  const int P0 = ws->P0, P1 = ws->P1;
+  strip_layers(S, a, moveI, m1, P0, P1);
+  move_strips(a, S, P0, P1, m.scratch);  // the snapshot is no longer needed
+  __syncthreads();
+  check_window_clear(a, P0, P1);
 }
 
 // Member of global block b: bpre holds the first block of every member (m + 1
@@ -1042,10 +1082,14 @@ struct YeeFixArgs {
 };
 
 // Orders every thread's earlier global and shared writes of the cluster
-// before its later reads (release / acquire at cluster scope).
+// before its later reads (release / acquire at cluster scope).  The runtime's
+// intrinsics, which the compiler keeps convergent, not inline assembly, which it
+// may copy into both sides of a divergent branch.
 __device__ __forceinline__ void cluster_barrier() {
   __threadfence();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();
+  __cluster_barrier_arrive();
+  __cluster_barrier_wait();
 }
 
 __device__ __forceinline__ int exchange_items(int L0, int L1, int which) {
@@ -1090,94 +1134,74 @@ __device__ __forceinline__ void yee_fixup(const FieldArgsT<T> &a, const YeeFixAr
   z.Ey = PlaneT<T>{x.z + zs - zoff, x.zpitch};
   z.Hx = PlaneT<T>{x.z + 2 * zs - zoff, x.zpitch};
   z.Hy = PlaneT<T>{x.z + 3 * zs - zoff, x.zpitch};
-  const int nw = L0 * L1;
   auto kind_of = [&](int i, int j) { return x.kind[(size_t)(j + 1) * x.kpitch + (i + 1)]; };
   auto cut_of = [&](uint8_t kd, int i, int j) -> const CutCellDev * {
     return kd == kKindCut ? a.cells + x.cutidx[(size_t)j * a.Nx + i] : nullptr;
   };
+  auto window = [&](auto &&cell) { for_cells<Sync::kRows>(L0, L1, tid, nth, [&](int c, int r) { cell(r * L0 + c, c, r); }); };
   // the box from the source set (cells off the stored planes read zero, as
   // the tile kernel's staging fills them)
-  {
-    const int nb = zw * zh;
-    for (int k = tid; k < 4 * nb; k += nth) {
-      const int p = k / nb, rem = k % nb, i = c0 - 1 + rem % zw, j = r0 - 1 + rem / zw;
-      const PlaneT<T> &src = p == 0 ? a.Ex : p == 1 ? a.Ey : p == 2 ? a.Hx : a.Hy;
-      const PlaneT<T> &dst = p == 0 ? z.Ex : p == 1 ? z.Ey : p == 2 ? z.Hx : z.Hy;
-      const bool stored = i >= -1 && i <= a.Nx && j >= -1 && j <= a.Ny;
-      dst.at(i, j) = stored ? src.at(i, j) : T(0);
-    }
-  }
+  for_cells<Sync::kRows>(zw, zh, tid, nth, [&](int c, int r) {
+    const int i = c0 - 1 + c, j = r0 - 1 + r;
+    const bool stored = i >= -1 && i <= a.Nx && j >= -1 && j <= a.Ny;
+    T v[4] = {T(0), T(0), T(0), T(0)};
+    if (stored) { v[0] = a.Ex.at(i, j); v[1] = a.Ey.at(i, j); v[2] = a.Hx.at(i, j); v[3] = a.Hy.at(i, j); }
+    z.Ex.at(i, j) = v[0]; z.Ey.at(i, j) = v[1]; z.Hx.at(i, j) = v[2]; z.Hy.at(i, j) = v[3];
+  });
   sync();
   // 1: half H, static [c0 - 1, c1) x [r0 - 1, r1 + 1), and the window
-  {
-    const int w = c1 - c0 + 1, ns = w * (r1 - r0 + 2);
-    for (int k = tid; k < ns + nw; k += nth) {
-      if (k >= ns) { window_h(a, k - ns); continue; }
-      const int i = c0 - 1 + k % w, j = r0 - 1 + k / w;
-      fix_h(a, z, kind_of(i, j), i, j, cut_of);
-    }
-  }
+  for_cells<Sync::kRows>(c1 - c0 + 1, r1 - r0 + 2, tid, nth, [&](int c, int r) {
+    const int i = c0 - 1 + c, j = r0 - 1 + r;
+    fix_h(a, z, kind_of(i, j), i, j, cut_of);
+  });
+  window([&](int, int i, int j) { window_h(a, i, j); });
   sync();
   for (int k = tid; k < exchange_items(L0, L1, 0); k += nth) exchange_body(z, 0, k);
   sync();
   // 2: Ex, static [c0 - 1, c1) x [r0, r1 + 1), and the window with the first push's current
-  {
-    const int w = c1 - c0 + 1, ns = w * (r1 - r0 + 1);
-    for (int k = tid; k < ns + nw; k += nth) {
-      if (k >= ns) { window_e<T, 0>(a, k - ns); continue; }
-      const int i = c0 - 1 + k % w, j = r0 + k / w;
-      const uint8_t kd = kind_of(i, j);
-      T e = z.Ex.at(i, j);
-      const T hx = z.Hx.at(i, j), hxm = z.Hx.at(i, j - 1), hy = z.Hy.at(i, j), hym = z.Hy.at(i, j - 1);
-      if (kd == kKindNone) continue;
-      ex_cell(a, kd, cut_of(kd, i, j), e, hx, hxm, hy, hym, x.zeroJ);
-      z.Ex.at(i, j) = e;
-    }
-  }
+  for_cells<Sync::kRows>(c1 - c0 + 1, r1 - r0 + 1, tid, nth, [&](int c, int r) {
+    const int i = c0 - 1 + c, j = r0 + r;
+    const uint8_t kd = kind_of(i, j);
+    T e = z.Ex.at(i, j);
+    const T hx = z.Hx.at(i, j), hxm = z.Hx.at(i, j - 1), hy = z.Hy.at(i, j), hym = z.Hy.at(i, j - 1);
+    if (kd == kKindNone) return;
+    ex_cell(a, kd, cut_of(kd, i, j), e, hx, hxm, hy, hym, x.zeroJ);
+    z.Ex.at(i, j) = e;
+  });
+  window([&](int k, int i, int j) { window_e<T, 0>(a, k, i, j); });
   sync();
   for (int k = tid; k < exchange_items(L0, L1, 1); k += nth) exchange_body(z, 1, k);
   sync();
   // 3: half H, static [c0 - 1, c1) x [r0, r1), and the window
-  {
-    const int w = c1 - c0 + 1, ns = w * (r1 - r0);
-    for (int k = tid; k < ns + nw; k += nth) {
-      if (k >= ns) { window_h(a, k - ns); continue; }
-      const int i = c0 - 1 + k % w, j = r0 + k / w;
-      fix_h(a, z, kind_of(i, j), i, j, cut_of);
-    }
-  }
+  for_cells<Sync::kRows>(c1 - c0 + 1, r1 - r0, tid, nth, [&](int c, int r) {
+    const int i = c0 - 1 + c, j = r0 + r;
+    fix_h(a, z, kind_of(i, j), i, j, cut_of);
+  });
+  window([&](int, int i, int j) { window_h(a, i, j); });
   sync();
   for (int k = tid; k < exchange_items(L0, L1, 0); k += nth) exchange_body(z, 0, k);
   sync();
-  // 4: static Ey on [c0, c1) x [r0, r1) (the window's Ey follows the second push)
-  {
-    const int w = c1 - c0, ns = w * (r1 - r0);
-    for (int k = tid; k < ns; k += nth) {
-      const int i = c0 + k % w, j = r0 + k / w;
-      const uint8_t kd = kind_of(i, j);
-      T e = z.Ey.at(i, j);
-      const T hx = z.Hx.at(i, j), hxl = z.Hx.at(i - 1, j), hy = z.Hy.at(i, j), hyl = z.Hy.at(i - 1, j);
-      if (kd == kKindNone) continue;
-      ey_cell(a, kd, cut_of(kd, i, j), e, hx, hxl, hy, hyl, x.zeroJ);
-      z.Ey.at(i, j) = e;
-    }
-  }
-  sync();
-  {
-    const int w = c1 - c0, nr = w * (r1 - r0);
-    for (int k = tid; k < 4 * nr; k += nth) {
-      const int p = k / nr, rem = k % nr, i = c0 + rem % w, j = r0 + rem / w;
-      const PlaneT<T> &src = p == 0 ? z.Ex : p == 1 ? z.Ey : p == 2 ? z.Hx : z.Hy;
-      const PlaneT<T> &dst = p == 0 ? x.out[0] : p == 1 ? x.out[1] : p == 2 ? x.out[2] : x.out[3];
-      dst.at(i, j) = src.at(i, j);
-    }
-  }
+  // 4: static Ey on [c0, c1) x [r0, r1) (the window's Ey follows the second
+  // push), and the region into the destination set: no cell reads another's Ey
+  for_cells<Sync::kRows>(c1 - c0, r1 - r0, tid, nth, [&](int c, int r) {
+    const int i = c0 + c, j = r0 + r;
+    const uint8_t kd = kind_of(i, j);
+    T e = z.Ey.at(i, j);
+    const T hx = z.Hx.at(i, j), hxl = z.Hx.at(i - 1, j), hy = z.Hy.at(i, j), hyl = z.Hy.at(i - 1, j);
+    if (kd != kKindNone) ey_cell(a, kd, cut_of(kd, i, j), e, hx, hxl, hy, hyl, x.zeroJ);
+    x.out[0].at(i, j) = z.Ex.at(i, j);
+    x.out[1].at(i, j) = e;
+    x.out[2].at(i, j) = hx;
+    x.out[3].at(i, j) = hy;
+  });
 }
 
 struct ClusterSync {
+  static constexpr bool kRows = false;
   __device__ __forceinline__ void operator()() const { cluster_barrier(); }
 };
 struct CtaSync {
+  static constexpr bool kRows = true;
   __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
 
@@ -1185,6 +1209,65 @@ template <class T>
 __global__ void __cluster_dims__(kFixCtas, 1, 1) __launch_bounds__(kFixThreads)
     k_yee_fixup(FieldArgsT<T> a, YeeFixArgs<T> x) {
   yee_fixup(a, x, (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x), ClusterSync{});
+}
+
+// The fix-up in one CTA with its scratch planes, the window's planes and the
+// cell kinds in shared memory: its phases pay no L2 round trip and no cluster
+// barrier (a 46 x 28 window in FP64: 11.3 us in a step's graph), but one SM does
+// all of it, so larger windows take the cluster (a 117 x 57 window in FP32: 67
+// us in one CTA, 28 on eight).
+template <class T>
+__host__ __device__ inline size_t fix_smem_bytes(int L0, int L1) {
+  const size_t z = (size_t)(L0 + 6) * (L1 + 7), w = (size_t)(L0 + 2) * (L1 + 2);
+  return 4 * (z + w) * sizeof(T) + (z + 15) / 16 * 16;
+}
+constexpr size_t kFixSmemMax = 224 * 1024;
+constexpr int kFixCtaCells = 2500;
+
+template <class T>
+__device__ __forceinline__ void yee_fixup_cta(const FieldArgsT<T> &a, const YeeFixArgs<T> &x, size_t smem_bytes) {
+  extern __shared__ __align__(16) uint8_t fix_smem[];
+  const int L0 = a.L0, L1 = a.L1, tid = threadIdx.x, nth = blockDim.x;
+  const int P0 = a.ws->P0, P1 = a.ws->P1;
+  if (fix_smem_bytes<T>(L0, L1) > smem_bytes || P0 < 1 || P1 < 1 || P0 + L0 >= a.Nx || P1 + L1 >= a.Ny) {
+    yee_fixup(a, x, tid, nth, CtaSync{});  // (off the mesh: it reports that and returns)
+    return;
+  }
+  const FixRegion R = fix_region(P0, P1, L0, L1, a.Nx, a.Ny);
+  const int zp = L0 + 6, np = (L0 + 2) * (L1 + 2);
+  const int zn = zp * (L1 + 7);
+  T *z = reinterpret_cast<T *>(fix_smem), *w = z + 4 * (size_t)zn;
+  uint8_t *kd = reinterpret_cast<uint8_t *>(w + 4 * (size_t)np);
+  FieldArgsT<T> b = a;
+  YeeFixArgs<T> y = x;
+  y.z = z; y.zpitch = zp; y.zrows = L1 + 7;
+  // kinds of the scratch box, at the fix-up's (j + 1) * kpitch + (i + 1)
+  y.kind = kd - ((ptrdiff_t)R.r0 * zp + R.c0);
+  y.kpitch = zp;
+  const int zw = R.c1 - R.c0 + 2, zh = R.r1 - R.r0 + 3;
+  for_cells<true>(zw, zh, tid, nth, [&](int c, int r) {
+    const int i = R.c0 - 1 + c, j = R.r0 - 1 + r;
+    kd[r * zp + c] = i <= a.Nx && j <= a.Ny ? x.kind[(size_t)(j + 1) * x.kpitch + (i + 1)] : (uint8_t)kKindNone;
+  });
+  b.mEx = PlaneT<T>{w, L0 + 2}; b.mEy = PlaneT<T>{w + np, L0 + 2};
+  b.mHx = PlaneT<T>{w + 2 * (size_t)np, L0 + 2}; b.mHy = PlaneT<T>{w + 3 * (size_t)np, L0 + 2};
+  for (int k = tid; k < np; k += nth) {
+    w[k] = a.mEx.p[k]; w[np + k] = a.mEy.p[k];
+    w[2 * np + k] = a.mHx.p[k]; w[3 * np + k] = a.mHy.p[k];
+  }
+  yee_fixup(b, y, tid, nth, CtaSync{});
+  // back: the window's Ex and H (its Ey waits for the second push)
+  for (int k = tid; k < np; k += nth) {
+    a.mEx.p[k] = w[k];
+    a.mHx.p[k] = w[2 * np + k]; a.mHy.p[k] = w[3 * np + k];
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kFixThreads, 1) k_yee_fixup_cta(const __grid_constant__ FieldArgsT<T> a,
+                                                                  const __grid_constant__ YeeFixArgs<T> x,
+                                                                  size_t smem_bytes) {
+  yee_fixup_cta(a, x, smem_bytes);
 }
 
 // The window's Ey sub-step with the second push's current, and the Ey strip
@@ -1195,7 +1278,7 @@ template <class T>
 __device__ __forceinline__ void window_ey_body(const FieldArgsT<T> &a, int k) {
   const int nw = a.L0 * a.L1;
   if (k < nw) {
-    window_e<T, 1>(a, k);
+    window_e<T, 1>(a, k, k % a.L0, k / a.L0);
     if (k % a.L0 == 0) exchange_body(a, 2, k / a.L0);
   } else if (k - nw < a.L1 + 2) {
     exchange_body(a, 2, a.L1 + (k - nw));
@@ -1209,20 +1292,27 @@ __global__ void __launch_bounds__(256) k_window_ey(FieldArgsT<T> a) {
 
 // --- the fused sweep of a batch of members: one persistent launch ------------
 //
-// A work queue (one counter, reset before the launch) hands out the items in
-// order: first every member's window fix-up (one CTA each, the longest
-// items), then every member's tiles.  Items do not depend on one another (a
-// tile reads the source set only, the fix-up writes cells no tile writes), so
-// no CTA waits for another; each staging wait is bounded (kErrStaging).
+// A work queue (one counter, reset before the launch) hands out every member's
+// tiles; the members' window fix-ups are a launch of their own beside it
+// (k_yee_fixup_batch).  Items do not depend on one another (a tile reads the
+// source set only, the fix-up writes cells no tile writes), so no CTA waits
+// for another; each staging wait is bounded (kErrStaging).
 template <class T>
 struct YeeBatchFix {
   FieldArgsT<T> a;   // static planes: the source set; the window; the first push's current
   YeeFixArgs<T> x;
 };
 
+// One CTA per member: 1024 threads on its window, where the queue's 256-thread
+// CTAs took longer for one fix-up than for all of a member's tiles.
 template <class T>
-__global__ void __launch_bounds__(256, 5) k_yee_batch(const YeeTileArgs<T> *targs, const YeeBatchFix<T> *fix,
-                                                      const int *tpre, int m, unsigned *queue) {
+__global__ void __launch_bounds__(kFixThreads, 1) k_yee_fixup_batch(const YeeBatchFix<T> *fix, size_t smem_bytes) {
+  yee_fixup_cta(fix[blockIdx.x].a, fix[blockIdx.x].x, smem_bytes);
+}
+
+template <class T>
+__global__ void __launch_bounds__(256, 5) k_yee_batch(const YeeTileArgs<T> *targs, const int *tpre, int m,
+                                                      unsigned *queue) {
   using G = YeeTile<T>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_ncut, s_item;
@@ -1233,7 +1323,7 @@ __global__ void __launch_bounds__(256, 5) k_yee_batch(const YeeTileArgs<T> *targ
     mbar_init(bar + 1, 1);
     mbar_init_fence();
   }
-  const int total = m + __ldg(tpre + m);
+  const int total = __ldg(tpre + m);
   uint32_t parity = 0;
   for (;;) {
     // the previous item's shared-memory reads and writes come before the
@@ -1242,13 +1332,8 @@ __global__ void __launch_bounds__(256, 5) k_yee_batch(const YeeTileArgs<T> *targ
     __syncthreads();
     if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
     __syncthreads();
-    const int item = s_item;
-    if (item >= total) break;
-    if (item < m) {
-      yee_fixup(fix[item].a, fix[item].x, (int)threadIdx.x, (int)blockDim.x, CtaSync{});
-      continue;
-    }
-    const int t = item - m;
+    const int t = s_item;
+    if (t >= total) break;
     int lo = 0, hi = m - 1;  // member of tile t
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -1259,6 +1344,118 @@ __global__ void __launch_bounds__(256, 5) k_yee_batch(const YeeTileArgs<T> *targ
     parity ^= 1u;
   }
 }
+
+// --- the end of a step: the window's Ey, its exchange and the window's move ---
+//
+// One cluster of six CTAs, a window plane each in shared memory: the Ey update
+// and its strip exchange, the move's shifted copy, the strips, the position
+// and the next push's set-up, in one launch (four before, 21 us and their gaps
+// of a step of 70 on a 46 x 28 window in FP64; now 7.5).
+constexpr int kTailCtas = 6, kTailThreads = 1024;
+
+// The next push's set-up at the end of a step (0: none).
+enum : int { kPrepNone = 0, kPrep64 = 1, kPrep32 = 2 };
+
+template <class T>
+__device__ __forceinline__ void step_tail(const FieldArgsT<T> &a, double h0, double h1, int prep, const PrepArgs &pa,
+                                          int f) {
+  extern __shared__ __align__(16) uint8_t tail_smem[];
+  __shared__ StripLayers S;
+  __shared__ MoveDecision s_move;
+  __shared__ int s_err;
+  T *sm = reinterpret_cast<T *>(tail_smem);
+  WinState *ws = a.ws;
+  const int L0 = a.L0, L1 = a.L1, W0 = L0 + 2, tid = threadIdx.x, nth = blockDim.x;
+  const int P0 = ws->P0, P1 = ws->P1;
+  if (tid == 0) {
+    s_err = *(volatile int *)&ws->err;
+    s_move = move_decision(ws, L0, L1);
+  }
+  const PlaneT<T> &mine = wplane_of(a, f);
+  const bool fresh = f == 1 || f == 5;  // Ey and Jy change before the move
+  for_cells<true>(W0, L1 + 2, tid, nth, [&](int c, int r) {
+    const int i = c - 1, j = r - 1, k = r * W0 + c;
+    T v = mine.p[k];
+    if (fresh && i >= 0 && i < L0 && j >= 0 && j < L1) {  // window_e<T, 1>, split over the two planes
+      const T J = (T)((double)(long long)a.acc[j * L0 + i] * a.acc_inv);
+      if (f == 5) v = J;
+      else
+        v = v - (a.key * (a.mHx.at(i, j) - a.mHx.at(i - 1, j) + a.mHy.at(i, j) - a.mHy.at(i - 1, j)) + a.dteps * J);
+    }
+    if (f == 1 && i == L0) {  // the exchange's static column right of the window
+      const int si = L0 + P0, sj = j + P1;
+      if (si >= 0 && si < a.Nx && sj >= 0 && sj < a.Ny) v = a.Ey.at(si, sj);
+    }
+    sm[k] = v;
+  });
+  cluster_barrier();  // every read of the window and of the current is done
+  const MoveDecision d = s_move;
+  const bool moved = s_err == 0 && d.ok && (d.moveI != 0 || d.dj != 0);
+  const int moveI = moved ? d.moveI : 0, m1 = moved ? d.dj : 0;
+  if (f == 5)
+    for (int k = tid; k < L0 * L1; k += nth) a.acc[k] = 0ull;
+  if (f == 1)
+    for (int j = tid; j < L1; j += nth) {  // the exchange's window column 0 -> static
+      const int si = P0, sj = j + P1;
+      if (si >= -1 && si <= a.Nx && sj >= -1 && sj <= a.Ny) a.Ey.at(si, sj) = sm[(j + 1) * W0 + 1];
+    }
+  if (moved || fresh) {
+    // the shifted copy over the reference's loop ranges (move_copy)
+    const int i0 = -moveI, i1 = L0 - 1;
+    int j0 = -(m1 > 0 ? m1 : 0), j1 = L1 - 1 - (m1 < 0 ? m1 : 0);
+    if (m1 == 0) { j0 -= 1; j1 += 1; }
+    for_cells<true>(W0, L1 + 2, tid, nth, [&](int c, int r) {
+      const int i = c - 1, j = r - 1, k = r * W0 + c;
+      const bool in = moved && i >= i0 && i <= i1 && j >= j0 && j <= j1;
+      if (in) mine.p[k] = sm[k + m1 * W0 + moveI];
+      else if (fresh) mine.p[k] = sm[k];
+    });
+  }
+  cluster_barrier();
+  const int Q0 = P0 + moveI, Q1 = P1 + m1;
+  // the bookkeeping in the second CTA, the strips in the first
+  if (f == 1 && tid == 0 && s_err == 0) {
+    if (!d.ok) set_err(ws, d.err);
+    else { ws->moves[0] = d.moveI; ws->moves[1] = d.dj; }
+    if (moved) {
+      ws->P0 = Q0; ws->P1 = Q1;
+      ws->mo0 += moveI * h0;
+      ws->mo1 += m1 * h1;
+    }
+  }
+  if (f == 0 && moved) {
+    strip_layers(S, a, moveI, m1, Q0, Q1);
+    move_strips(a, S, Q0, Q1, sm);
+    check_window_clear(a, Q0, Q1);
+  }
+  if (f == 1 && prep != kPrepNone && tid == 0) {
+    if (prep == kPrep32) prep32_body(ws, 2, true);
+    else push_prep_body(ws, pa.h0, pa.h1, pa.em0, pa.em2, pa.cm0, true);
+  }
+}
+
+template <class T>
+__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads, 1)
+    k_step_tail(const __grid_constant__ FieldArgsT<T> a, double h0, double h1, int prep, PrepArgs pa) {
+  step_tail(a, h0, h1, prep, pa, (int)blockIdx.x);
+}
+
+// The same for a batch: one cluster per member.
+template <class T>
+__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(kTailThreads, 1)
+    k_step_tail_batch(const FieldArgsT<T> *ey, const MoveArgs<T> *mv) {
+  const int m = blockIdx.x / kTailCtas;
+  step_tail(ey[m], mv[m].h0, mv[m].h1, kPrepNone, PrepArgs{}, (int)(blockIdx.x % kTailCtas));
+}
+
+// Shared memory of a CTA of the tail: a window plane, or the strips' values if
+// they are more (twelve layers at most).
+template <class T>
+static size_t tail_smem_bytes(int L0, int L1) {
+  const size_t np = (size_t)(L0 + 2) * (L1 + 2), strips = 6 * (size_t)(L0 + L1 + 4);
+  return (np > strips ? np : strips) * sizeof(T);
+}
+constexpr size_t kTailSmemMax = 220 * 1024;
 
 template <class T>
 __global__ void __launch_bounds__(256) k_window_ey_batch(const FieldArgsT<T> *args, const int *bpre, int m) {
@@ -1517,7 +1714,7 @@ static void fill_fix_args(YeeFixArgs<T> &x, const PlaneT<T> *dst, const uint8_t 
 template <class T>
 int launch_yee_fused(const FieldArgsT<T> &a, const PlaneT<T> *dst, const uint8_t *kind, int kpitch,
                      const int *cutidx, T *z, int zpitch, int zrows, long long spin, cudaStream_t s, cudaStream_t s2,
-                     cudaEvent_t fork, cudaEvent_t join) {
+                     cudaEvent_t fork) {
   using G = YeeTile<T>;
   if (zpitch < a.L0 + 6 || zrows < a.L1 + 7) return kErrArg;
   YeeTileArgs<T> t;
@@ -1529,11 +1726,19 @@ int launch_yee_fused(const FieldArgsT<T> &a, const PlaneT<T> *dst, const uint8_t
   YeeFixArgs<T> x;
   fill_fix_args(x, dst, kind, kpitch, cutidx, z, zpitch, zrows);
   // the tiles and the fix-up write disjoint cells and read only the source
-  // set: the fix-up runs on s2 beside the tiles, s waits for both
+  // set: the fix-up runs on s2 beside the tiles.  s does not wait for it here:
+  // the second push needs the window only and follows it on s2.
   if (cudaEventRecord(fork, s) != cudaSuccess || cudaStreamWaitEvent(s2, fork, 0) != cudaSuccess) return kErrCuda;
-  k_yee_fixup<T><<<kFixCtas, kFixThreads, 0, s2>>>(a, x);
+  const size_t fb = fix_smem_bytes<T>(a.L0, a.L1);
+  if (fb <= kFixSmemMax && a.L0 * a.L1 <= kFixCtaCells) {
+    if (cudaFuncSetAttribute(k_yee_fixup_cta<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmemMax) !=
+        cudaSuccess)
+      return kErrCuda;
+    k_yee_fixup_cta<T><<<1, kFixThreads, fb, s2>>>(a, x, fb);
+  } else {
+    k_yee_fixup<T><<<kFixCtas, kFixThreads, 0, s2>>>(a, x);
+  }
   k_yee_tiles<T><<<t.tilesX * tilesY, G::THREADS, G::SMEM, s>>>(t);
-  if (cudaEventRecord(join, s2) != cudaSuccess || cudaStreamWaitEvent(s, join, 0) != cudaSuccess) return kErrCuda;
   return kOk;
 }
 
@@ -1541,6 +1746,32 @@ template <class T>
 void launch_window_ey(const FieldArgsT<T> &a, cudaStream_t s) {
   const int n = a.L0 * a.L1 + a.L1 + 2;
   k_window_ey<T><<<(n + 255) / 256, 256, 0, s>>>(a);
+}
+
+template <class T>
+int launch_step_tail(const FieldArgsT<T> &a, double h0, double h1, int order, cudaStream_t s) {
+  const size_t sb = tail_smem_bytes<T>(a.L0, a.L1);
+  if (sb > kTailSmemMax) return 0;
+  if (cudaFuncSetAttribute(k_step_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  k_step_tail<T><<<kTailCtas, kTailThreads, sb, s>>>(a, h0, h1, sizeof(T) == 4 ? kPrep32 : kPrep64,
+                                                     prep_args(a.ws, h0, h1, order));
+  return 1;
+}
+
+template <class T>
+size_t step_tail_smem(int L0, int L1) {
+  const size_t sb = tail_smem_bytes<T>(L0, L1);
+  return sb <= kTailSmemMax ? sb : 0;
+}
+
+template <class T>
+void launch_step_tail_batch(const FieldArgsT<T> *ey, const MoveArgs<T> *mv, int m, size_t smem, cudaStream_t s) {
+  cudaFuncSetAttribute(k_step_tail_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemMax);
+  k_step_tail_batch<T><<<kTailCtas * m, kTailThreads, smem, s>>>(ey, mv);
 }
 
 template <class T>
@@ -1564,16 +1795,27 @@ int yee_batch_entry(const FieldArgsT<T> &a, const PlaneT<T> *dst, const uint8_t 
 }
 
 template <class T>
-int launch_yee_batch(const void *targs, const void *fix, const int *tpre, int m, unsigned *queue, cudaStream_t s) {
+size_t fixup_smem(int L0, int L1) {
+  const size_t fb = fix_smem_bytes<T>(L0, L1);
+  return fb <= kFixSmemMax ? fb : 0;
+}
+
+template <class T>
+int launch_yee_batch(const void *targs, const void *fix, const int *tpre, int m, size_t fix_smem, unsigned *queue,
+                     cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join) {
   using G = YeeTile<T>;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaFuncSetAttribute(k_yee_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_yee_fixup_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFixSmemMax) !=
+          cudaSuccess ||
       cudaMemsetAsync(queue, 0, sizeof(unsigned), s) != cudaSuccess)
     return kErrCuda;
-  k_yee_batch<T><<<5 * sms, G::THREADS, G::SMEM, s>>>(static_cast<const YeeTileArgs<T> *>(targs),
-                                                        static_cast<const YeeBatchFix<T> *>(fix), tpre, m, queue);
+  if (cudaEventRecord(fork, s) != cudaSuccess || cudaStreamWaitEvent(s2, fork, 0) != cudaSuccess) return kErrCuda;
+  k_yee_fixup_batch<T><<<m, kFixThreads, fix_smem, s2>>>(static_cast<const YeeBatchFix<T> *>(fix), fix_smem);
+  k_yee_batch<T><<<5 * sms, G::THREADS, G::SMEM, s>>>(static_cast<const YeeTileArgs<T> *>(targs), tpre, m, queue);
+  if (cudaEventRecord(join, s2) != cudaSuccess || cudaStreamWaitEvent(s, join, 0) != cudaSuccess) return kErrCuda;
   return kOk;
 }
 
@@ -1610,12 +1852,17 @@ void launch_build_kind(const uint8_t *mask, const int *cutidx, int Nx, int Ny, u
   template void launch_exchange_batch<T>(const FieldArgsT<T> *, const int *, int, int, int, cudaStream_t); \
   template void launch_move_batch<T>(const MoveArgs<T> *, int, cudaStream_t);                        \
   template int launch_yee_fused<T>(const FieldArgsT<T> &, const PlaneT<T> *, const uint8_t *, int, const int *, T *, \
-                                   int, int, long long, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t); \
+                                   int, int, long long, cudaStream_t, cudaStream_t, cudaEvent_t);           \
   template void launch_window_ey<T>(const FieldArgsT<T> &, cudaStream_t);                            \
   template size_t yee_batch_bytes<T>(int);                                                          \
   template int yee_batch_entry<T>(const FieldArgsT<T> &, const PlaneT<T> *, const uint8_t *, int, const int *, T *, \
                                   int, int, long long, void *, void *, int *);                      \
-  template int launch_yee_batch<T>(const void *, const void *, const int *, int, unsigned *, cudaStream_t); \
+  template int launch_yee_batch<T>(const void *, const void *, const int *, int, size_t, unsigned *, cudaStream_t, \
+                                   cudaStream_t, cudaEvent_t, cudaEvent_t);                         \
+  template size_t fixup_smem<T>(int, int);                                                          \
+  template int launch_step_tail<T>(const FieldArgsT<T> &, double, double, int, cudaStream_t);        \
+  template size_t step_tail_smem<T>(int, int);                                                      \
+  template void launch_step_tail_batch<T>(const FieldArgsT<T> *, const MoveArgs<T> *, int, size_t, cudaStream_t); \
   template void launch_window_ey_batch<T>(const FieldArgsT<T> *, const int *, int, int, cudaStream_t);
 CSRST_FIELDS_INSTANTIATE(double)
 CSRST_FIELDS_INSTANTIATE(float)

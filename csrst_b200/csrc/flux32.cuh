@@ -56,6 +56,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include "sinkbox.cuh"
+
 namespace csrst {
 
 template <int ORDER>
@@ -302,15 +304,6 @@ __device__ __forceinline__ void emit_row(Sink &s, int i0, int j, const long long
   for (int c = 0; c < N; ++c)
     if (v[c] != 0) s(i0 + c, j, v[c]);
 }
-// Tells a sink that wants to know the box its rows will lie in.
-template <int NX, int NY, class Sink>
-__device__ __forceinline__ auto open_box(Sink &s, int i0, int j0, int)
-    -> decltype(s.template box<NX, NY>(i0, j0), void()) {
-  s.template box<NX, NY>(i0, j0);
-}
-template <int NX, int NY, class Sink>
-__device__ __forceinline__ void open_box(Sink &, int, int, long) {}
-
 // The displacement of a move, from its exact end points in FP64 (a difference
 // of O(1) FP32 coordinates would carry an absolute error of their ulp).
 __device__ __forceinline__ float displacement(int dc, float b, float a) {

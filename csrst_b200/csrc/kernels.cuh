@@ -4,6 +4,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "shapes.cuh"
 
 namespace csrst {
 
@@ -19,9 +20,12 @@ struct PushArgs {
   unsigned long long *acc;  // L0 * L1 fixed-point current for jcomp
   double acc_scale;
   int jcomp, pending;
+  int narrow;                // every |contribution * acc_scale| < 2^51
+  int prep_next;             // set up the next push's gather patches at the end (launch_push)
+  int em0, em2, cm0;         // their margins (PrepArgs)
   double half;               // 0.5 * dt * c
   double fact1, fact2;       // half * q/m, fact1 * c
-  double h0, h1, dt;
+  DepositScale ds;
   // hard-edge dipole (Bend::getExternalField, Bend.cpp:865-907)
   double bz, Lb, hw, chh, shh, bwidth;
 };
@@ -122,8 +126,11 @@ void launch_push_batch(const PushGroup *groups, int ngroups, int m, int grid, co
 void launch_bbox_next(const double *x, const double *y, const double *px, const double *py, long long n,
                       double half, int pending, WinState *ws, cudaStream_t s);
 void launch_push_prep(WinState *ws, double h0, double h1, int order, cudaStream_t s);
+constexpr int kPushCtas = 2;  // CTAs per SM of launch_push
+// fills ds and the gather-patch margins
+void set_push_consts(PushArgs &a, int order, double h0, double h1, double dt);
+// push, box swap, deposit bounds and, when a.prep_next, the next push's set-up
 void launch_push(const PushArgs &a, int order, int grid, cudaStream_t s);
-void launch_global_bounds(WinState *ws, double h0, double h1, cudaStream_t s);
 void launch_drift(double *x, double *y, const double *px, const double *py, long long n, double full,
                   cudaStream_t s);
 void launch_gather(int order, int comp, const double *patch, int nx, double o0, double o1, double h0,
@@ -159,18 +166,18 @@ template <class T> void launch_move_batch(const MoveArgs<T> *args, int m, cudaSt
 // window, its first push's current and that component's acc_inv.  kind: the
 // cell-kind map (static storage layout, kpitch bytes per row, a multiple of
 // 16); z: 4 scratch planes of zpitch >= L0 + 6 by zrows >= L1 + 7 elements;
-// spin: polls of a tile's staging wait.  The window fix-up runs on s2
-// between the events fork (recorded on s) and join (s waits for it).
+// spin: polls of a tile's staging wait.  The window fix-up runs on s2 after
+// the event fork (recorded on s); s does not wait for s2.
 // Returns kOk, or kErrArg / kErrCuda (tensor-map set-up) before anything is
 // launched.
 template <class T>
 int launch_yee_fused(const FieldArgsT<T> &a, const PlaneT<T> *dst, const uint8_t *kind, int kpitch,
                      const int *cutidx, T *z, int zpitch, int zrows, long long spin, cudaStream_t s, cudaStream_t s2,
-                     cudaEvent_t fork, cudaEvent_t join);
+                     cudaEvent_t fork);
 // The window's Ey sub-step after the second push, with its strip exchange.
 template <class T> void launch_window_ey(const FieldArgsT<T> &a, cudaStream_t s);
 // The fused sweep of a batch of members as one persistent launch over a work
-// queue: yee_batch_bytes(0 / 1) is the size of one member's entry in the tile
+// queue of tiles, with the window fix-ups (one CTA per member) beside it on s2: yee_batch_bytes(0 / 1) is the size of one member's entry in the tile
 // / fix-up table, yee_batch_entry fills a member's entries (host memory; the
 // arguments as for launch_yee_fused) and its tile count, launch_yee_batch
 // resets the queue counter and launches over the device tables (tpre: first
@@ -181,7 +188,21 @@ template <class T>
 int yee_batch_entry(const FieldArgsT<T> &a, const PlaneT<T> *dst, const uint8_t *kind, int kpitch, const int *cutidx,
                     T *z, int zpitch, int zrows, long long spin, void *tile_out, void *fix_out, int *ntiles);
 template <class T>
-int launch_yee_batch(const void *targs, const void *fix, const int *tpre, int m, unsigned *queue, cudaStream_t s);
+int launch_yee_batch(const void *targs, const void *fix, const int *tpre, int m, size_t fix_smem, unsigned *queue,
+                     cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join);
+// Shared memory of one window's fix-up (0: it runs on global memory); a batch
+// launches with the largest of its members'.
+template <class T> size_t fixup_smem(int L0, int L1);
+// The end of a step in one launch: the window's Ey and its exchange (a: its
+// second-push arguments), the window move and the next push's set-up.  Returns
+// 0, with nothing launched, for a window plane larger than shared memory
+// (launch_window_ey and launch_move then, and no set-up).
+template <class T> int launch_step_tail(const FieldArgsT<T> &a, double h0, double h1, int order, cudaStream_t s);
+// The same over a batch without the set-up: smem the largest step_tail_smem of
+// its members, none of them 0.
+template <class T> size_t step_tail_smem(int L0, int L1);
+template <class T>
+void launch_step_tail_batch(const FieldArgsT<T> *ey, const MoveArgs<T> *mv, int m, size_t smem, cudaStream_t s);
 template <class T>
 void launch_window_ey_batch(const FieldArgsT<T> *args, const int *bpre, int m, int nblocks, cudaStream_t s);
 void launch_build_kind(const uint8_t *mask, const int *cutidx, int Nx, int Ny, uint8_t *kind, int kpitch,

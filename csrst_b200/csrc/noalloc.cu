@@ -38,6 +38,7 @@ __global__ void k_noalloc_deposit(int comp, const double *ox, const double *oy, 
                                   const double *y, const double *q, long long n, double org0, double org1,
                                   double h0, double h1, double dt, int i0, int j0, int ni, int nj,
                                   unsigned long long *acc, double scale) {
+  const DepositScale ds = deposit_scale<ORDER>(h0, h1, dt);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     bool dropped = false;
@@ -48,7 +49,7 @@ __global__ void k_noalloc_deposit(int comp, const double *ox, const double *oy, 
       if (!in && iv != 0) dropped = true;
       warp_add(acc, in ? b * ni + a : -1, iv);
     };
-    if (!deposit_particle<ORDER>(comp, q[i], ox[i], oy[i], x[i], y[i], org0, org1, h0, h1, h0, h1, dt, sink))
+    if (!deposit_particle<ORDER>(comp, q[i], ox[i], oy[i], x[i], y[i], org0, org1, ds, sink))
       g_noalloc_err[0] = kErrCrossings;
     if (dropped) g_noalloc_err[1] = 1;
   }

@@ -19,6 +19,7 @@
 #include "accum.cuh"
 #include "bbox.cuh"
 #include "kernels.cuh"
+#include "pushwork.cuh"
 #include "shapes.cuh"
 
 namespace csrst {
@@ -46,60 +47,66 @@ __global__ void k_bbox_clear(WinState *ws, int slot) {
   if (threadIdx.x == 0) bbox_reset(ws->bb[slot < 0 ? ws->cur : slot]);
 }
 
-// Before a push: derive the gather patches from the particle box of the
-// positions the push will gather at (PartBunch::getLocalPDomain and
-// getFields), and reset the accumulators the push will fill.
-// em: getExtraMarginEdge (x first, x last, y first, y last); cm: getExtraMarginCell.
-__device__ __forceinline__ void push_prep_body(WinState *ws, double h0, double h1, int em0, int em2, int cm0) {
-  const int c = ws->cur;
-  const double mn0 = ord_dbl(ws->bb[c][0]), mn1 = ord_dbl(ws->bb[c][1]);
-  const double mx0 = ord_dbl(ws->bb[c][2]), mx1 = ord_dbl(ws->bb[c][3]);
-  int lp[4];
-  if (mn0 <= mx0) {
-    lp[0] = (int)floor((mn0 - ws->mo0) / h0); lp[1] = (int)floor((mx0 - ws->mo0) / h0);
-    lp[2] = (int)floor((mn1 - ws->mo1) / h1); lp[3] = (int)floor((mx1 - ws->mo1) / h1);
-  } else {  // no particles: PartBunch::getLocalPDomain with Rmin = Rmax = 0
-    lp[0] = lp[1] = (int)floor((0.0 - ws->mo0) / h0);
-    lp[2] = lp[3] = (int)floor((0.0 - ws->mo1) / h1);
+__global__ void k_push_prep(PrepArgs p) {
+  if (threadIdx.x == 0) push_prep_body(p.ws, p.h0, p.h1, p.em0, p.em2, p.cm0, false);
+}
+
+// After the last push of a step: the deposit's particle bounds relative to
+// the window (PartBunch::getLocalPDomainInclOld -> setGlobalBounds).
+__device__ __forceinline__ void global_bounds_body(WinState *ws, double h0, double h1) {
+  const double mn0 = ord_dbl(ws->bball[0]), mn1 = ord_dbl(ws->bball[1]);
+  const double mx0 = ord_dbl(ws->bball[2]), mx1 = ord_dbl(ws->bball[3]);
+  if (!(mn0 <= mx0)) { ws->gb[0] = 0; ws->gb[1] = -1; ws->gb[2] = 0; ws->gb[3] = -1; return; }
+  ws->gb[0] = (int)floor((mn0 - ws->mo0) / h0);
+  ws->gb[1] = (int)floor((mx0 - ws->mo0) / h0);
+  ws->gb[2] = (int)floor((mn1 - ws->mo1) / h1);
+  ws->gb[3] = (int)floor((mx1 - ws->mo1) / h1);
+}
+
+// Rounds a contribution to the fixed-point unit and adds it to the tile.
+// narrow (uniform over the launch): every |v * scale| < 2^51, so that the
+// rounded integer is the low mantissa bits of v * scale + 1.5 * 2^52, one FP64
+// add, where the conversion instruction runs at an eighth of its rate.
+template <class Tile>
+struct FixedSink {
+  TileSink<Tile> t;
+  double scale;
+  bool narrow;
+  template <int NX, int NY>
+  __device__ __forceinline__ void box(int i, int j) { t.template box<NX, NY>(i, j); }
+  __device__ __forceinline__ void operator()(int i, int j, double v) {
+    const double x = v * scale;
+    const long long k = narrow ? __double_as_longlong(x + 6755399441055744.0) - 0x4338000000000000ll
+                               : __double2ll_rn(x);
+    t.one(i, j, k);
   }
-  for (int k = 0; k < 4; ++k) ws->lp[k] = lp[k];
-  // Every gather tap lies within [lp - 2, lp + 2] (the cubic edge stencil
-  // reaches furthest); the window planes hold one guard cell.  A bunch that
-  // no longer fits stops the run instead of reading outside the window.
-  if (mn0 <= mx0 && (lp[0] - 2 < -1 || lp[1] + 2 > ws->L0 || lp[2] - 2 < -1 || lp[3] + 2 > ws->L1))
-    set_err(ws, kErrWindowFit);
-  const double po0 = ws->mo0 + lp[0] * h0, po1 = ws->mo1 + lp[2] * h1;
-  ws->hz_o0 = po0 + cm0 * h0; ws->hz_o1 = po1 + cm0 * h1;
-  ws->ex_o0 = po0 + em0 * h0; ws->ex_o1 = po1 + em2 * h1;
-  ws->ey_o0 = po0 + em2 * h0; ws->ey_o1 = po1 + em0 * h1;
-  ws->hz_I = lp[0] + cm0; ws->hz_J = lp[2] + cm0;
-  ws->ex_I = lp[0] + em0; ws->ex_J = lp[2] + em2;
-  ws->ey_I = lp[0] + em2; ws->ey_J = lp[2] + em0;
-  bbox_reset(ws->bb[1 - c]);
-  bbox_reset(ws->bball);
+};
+
+// The few moves that cross more borders: a call of its own, so that the code
+// of the crossing list (an array in local memory) stays out of the push's loop.
+template <int ORDER, int COMP, class Tile>
+__device__ __noinline__ bool deposit_general(double q, double ao0, double ao1, double an0, double an1, double org0,
+                                             double org1, DepositScale ds, FixedSink<Tile> sink) {
+  return deposit_move<ORDER, true>(COMP, q, ao0, ao1, an0, an1, org0, org1, ds, sink);
 }
 
-__global__ void k_push_prep(WinState *ws, double h0, double h1, int em0, int em2, int cm0) {
-  if (threadIdx.x == 0) push_prep_body(ws, h0, h1, em0, em2, cm0);
-}
-
-// After a push: flip the bbox slot.
-__global__ void k_push_post(WinState *ws) {
-  if (threadIdx.x == 0) ws->cur = 1 - ws->cur;
+// The stored state of a particle, read one round ahead of its move.
+struct In64 {
+  double x, y, p0, p1, q;
+};
+__device__ __forceinline__ In64 load64(const PushArgs &a, long long i) {
+  return In64{__ldcs(a.x + i), __ldcs(a.y + i), __ldcs(a.px + i), __ldcs(a.py + i), __ldg(a.q + i)};
 }
 
 // Dynamic shared memory: [window accumulator (SMEM only)][per-thread deposit tiles].
-// One CTA's share [beg, end) of one push.  All threads of the CTA call it
-// together; it ends with a barrier, so a CTA can run it for several members
-// in turn.
-template <int ORDER, bool SMEM>
-__device__ __forceinline__ void push_body(const PushArgs &a, long long beg, long long end, PushShared &sh,
+// One CTA's share of one push.  All threads of the CTA call it together; it
+// ends with a barrier, so a CTA can run it for several members in turn.
+template <int ORDER, int COMP, bool SMEM, class Work>
+__device__ __forceinline__ void push_body(const PushArgs &a, const Work &work, PushShared &sh,
                                           unsigned long long *sacc) {
   int *tb = sh.tb;  // touched box of this CTA (window cells)
+  if (entry_error(a.ws, sh)) return;  // the whole CTA leaves together
   WinState *ws = a.ws;
-  if (threadIdx.x == 0) sh.err = *(volatile int *)&ws->err;
-  __syncthreads();
-  if (sh.err) return;  // the whole CTA leaves together
   const int L0 = ws->L0, L1 = ws->L1;
   const int ncell = L0 * L1;
   using Tile = typename TileFor<ORDER>::T;
@@ -107,14 +114,13 @@ __device__ __forceinline__ void push_body(const PushArgs &a, long long beg, long
   unsigned long long *tmem = SMEM ? sacc + ncell : sacc;
   if (SMEM)
     for (int k = threadIdx.x; k < ncell; k += blockDim.x) sacc[k] = 0ull;
-  for (int k = threadIdx.x; k < Tile::kSize * (int)blockDim.x; k += blockDim.x) tmem[k] = 0ull;
+  for (int k = threadIdx.x; k < Tile::kSize * kPushThreads; k += kPushThreads) tmem[k] = 0ull;
   if (threadIdx.x == 0) { tb[0] = L0; tb[1] = L1; tb[2] = -1; tb[3] = -1; }
   __syncthreads();
   Tile tile;
   tile.init(tmem, L0, L1);
   const double mo0 = ws->mo0, mo1 = ws->mo1;
-  const double h0 = a.h0, h1 = a.h1;
-  const double ood0 = 1.0 / h0, ood1 = 1.0 / h1;
+  const DepositScale &ds = a.ds;
   const int wp = a.wpitch;
   // Patch views: relative (0,0) is absolute window index (I, J); the window
   // plane stores absolute (i, j) at (j + 1) * wp + (i + 1).
@@ -127,72 +133,89 @@ __device__ __forceinline__ void push_body(const PushArgs &a, long long beg, long
 
   double amn0 = INFINITY, amn1 = INFINITY, amx0 = -INFINITY, amx1 = -INFINITY;  // R0 u R2
   double bmn0 = INFINITY, bmn1 = INFINITY, bmx0 = -INFINITY, bmx1 = -INFINITY;  // next R1
+  auto lower = [](double &m, double v) { m = v < m ? v : m; };
+  auto upper = [](double &m, double v) { m = v > m ? v : m; };
   bool overflow = false;
-  const double scale = a.acc_scale;
-  auto sink = [&](int i, int j, double v) { tile.template add<SMEM>(i, j, __double2ll_rn(v * scale), win, L0, L1); };
 
-  // The CTA owns a contiguous slice of the (cell-ordered) particles.  The
-  // rounds are the same for every lane, so that the warp re-bases its
+  // The rounds are the same for every lane, so that the warp re-bases its
   // deposit tile together.
-  const long long rounds = end > beg ? (end - beg + blockDim.x - 1) / blockDim.x : 0;
-  for (long long it = 0; it < rounds; ++it) {
-    const long long i = beg + it * blockDim.x + threadIdx.x;
-    bool ok = i < end;
-    double x = 0.0, y = 0.0, p0 = 0.0, p1 = 0.0, q = 0.0, r0x = 0.0, r0y = 0.0, w0 = 0.0, w1 = 0.0;
-    if (ok) {
-      x = a.x[i]; y = a.y[i]; p0 = a.px[i]; p1 = a.py[i]; q = a.q[i];
-      if (!(isfinite(x) && isfinite(y) && isfinite(p0) && isfinite(p1))) {
+  const int lane = threadIdx.x & 31;
+  long long n0, end, step;
+  for (int k = 0; work.run(k, n0, end, step); ++k) {
+    In64 next{};
+    if (n0 + lane < end) next = load64(a, n0 + lane);
+    for (; n0 < end; n0 += step) {
+      const long long i = n0 + lane;
+      const In64 cur = next;
+      if (i + step < end) next = load64(a, i + step);
+      bool ok = i < end;
+      double x = cur.x, y = cur.y, p0 = cur.p0, p1 = cur.p1, r0x = 0.0, r0y = 0.0, w0 = 0.0, w1 = 0.0;
+      if (ok && !(isfinite(x) && isfinite(y) && isfinite(p0) && isfinite(p1))) {
         set_err(ws, kErrWindowFit);
         ok = false;
       }
-    }
-    if (ok) {
-      double r = inv_gamma(p0, p1);
-      w0 = a.half * p0 * r; w1 = a.half * p1 * r;
-      if (a.pending) { x = x + (-w0); y = y + (-w1); }          // drift_particles(-dt/2)
-      r0x = x; r0y = y;                                          // oldR
-      x = x + w0; y = y + w1;                                    // R1
-      // gather (FieldPatch::gather x3; Hz = Hzx + Hzy on the fly)
-      const double E0 = gather_edge<ORDER>(pex, (x - exo0) * ood0, (y - exo1) * ood1, 0);
-      const double E1 = gather_edge<ORDER>(pey, (x - eyo0) * ood0, (y - eyo1) * ood1, 1);
-      const double hpp0 = (x - hzo0) * ood0, hpp1 = (y - hzo1) * ood1;
-      const double Hf = gather_cell<ORDER>(SumView{phx, phy}, hpp0, hpp1);
-      // hard-edge dipole
-      const double D0 = x - a.Lb, D1 = y - a.hw;
-      const double dist = a.chh * D0 - a.shh * D1;
-      const double bext = (dist > 0.0 && dist < a.bwidth) ? a.bz : 0.0;
-      const double B = kMu0 * Hf + 0.5 * bext;
-      // kick + rotation (PartBunch.cpp:366-383)
-      const double k0 = a.fact1 * E0, k1 = a.fact1 * E1;
-      double u0 = p0 + k0, u1 = p1 + k1;
-      const double aa = a.fact2 * B * inv_gamma(u0, u1);
-      const double s0 = u0 + aa * u1, s1 = u1 + aa * (-u0);
-      const double tmp = 1.0 + aa * aa;
-      u0 = ((1.0 + aa * aa) * s0 + aa * s1) / tmp;
-      u1 = ((1.0 + aa * aa) * s1 - aa * s0) / tmp;
-      p0 = u0 + k0; p1 = u1 + k1;
-      r = inv_gamma(p0, p1);
-      w0 = a.half * p0 * r; w1 = a.half * p1 * r;
-      x = x + w0; y = y + w1;                                    // R2
-      a.x[i] = x; a.y[i] = y; a.px[i] = p0; a.py[i] = p1;
-    }
-    // current deposit R0 -> R2 in window coordinates, summed in the warp's tile
-    tile.template rebase<SMEM>(ok, ok ? (int)floor((r0x - mo0) * ood0) : 0, ok ? (int)floor((r0y - mo1) * ood1) : 0,
-                               win, L0, L1);
-    if (ok) {
-      if (!deposit_particle<ORDER>(a.jcomp, q, r0x, r0y, x, y, mo0, mo1, h0, h1, h0, h1, a.dt, sink))
-        overflow = true;
-      amn0 = fmin(amn0, fmin(x, r0x)); amn1 = fmin(amn1, fmin(y, r0y));
-      amx0 = fmax(amx0, fmax(x, r0x)); amx1 = fmax(amx1, fmax(y, r0y));
-      // next push gathers at (R2 - h v) + h v
-      const double nx = (x + (-w0)) + w0, ny = (y + (-w1)) + w1;
-      bmn0 = fmin(bmn0, nx); bmn1 = fmin(bmn1, ny); bmx0 = fmax(bmx0, nx); bmx1 = fmax(bmx1, ny);
+      if (ok) {
+        double r = inv_gamma(p0, p1);
+        w0 = a.half * p0 * r; w1 = a.half * p1 * r;
+        if (a.pending) { x = x + (-w0); y = y + (-w1); }          // drift_particles(-dt/2)
+        r0x = x; r0y = y;                                          // oldR
+        x = x + w0; y = y + w1;                                    // R1
+        // gather (FieldPatch::gather x3; Hz = Hzx + Hzy on the fly)
+        const double E0 = gather_edge<ORDER>(pex, (x - exo0) * ds.ood0, (y - exo1) * ds.ood1, 0);
+        const double E1 = gather_edge<ORDER>(pey, (x - eyo0) * ds.ood0, (y - eyo1) * ds.ood1, 1);
+        const double hpp0 = (x - hzo0) * ds.ood0, hpp1 = (y - hzo1) * ds.ood1;
+        const double Hf = gather_cell<ORDER>(SumView{phx, phy}, hpp0, hpp1);
+        // hard-edge dipole
+        const double D0 = x - a.Lb, D1 = y - a.hw;
+        const double dist = a.chh * D0 - a.shh * D1;
+        const double bext = (dist > 0.0 && dist < a.bwidth) ? a.bz : 0.0;
+        const double B = kMu0 * Hf + 0.5 * bext;
+        // kick + rotation (PartBunch.cpp:366-383)
+        const double k0 = a.fact1 * E0, k1 = a.fact1 * E1;
+        double u0 = p0 + k0, u1 = p1 + k1;
+        const double aa = a.fact2 * B * inv_gamma(u0, u1);
+        const double s0 = u0 + aa * u1, s1 = u1 + aa * (-u0);
+        const double tmp = 1.0 + aa * aa;
+        u0 = ((1.0 + aa * aa) * s0 + aa * s1) / tmp;
+        u1 = ((1.0 + aa * aa) * s1 - aa * s0) / tmp;
+        p0 = u0 + k0; p1 = u1 + k1;
+        r = inv_gamma(p0, p1);
+        w0 = a.half * p0 * r; w1 = a.half * p1 * r;
+        x = x + w0; y = y + w1;                                    // R2
+        a.x[i] = x; a.y[i] = y; a.px[i] = p0; a.py[i] = p1;
+      }
+      // current deposit R0 -> R2 in window coordinates, summed in the warp's tile
+      tile.template rebase<SMEM>(ok, ok ? (int)floor((r0x - mo0) * ds.ood0) : 0,
+                                 ok ? (int)floor((r0y - mo1) * ds.ood1) : 0, win, L0, L1);
+      if (ok) {
+        bool fits;
+        if constexpr (SMEM) {
+          const double scale = a.acc_scale;
+          auto sink = [&](int si, int sj, double v) {
+            tile.template add<true>(si, sj, __double2ll_rn(v * scale), win, L0, L1);
+          };
+          fits = deposit_particle<ORDER>(COMP, cur.q, r0x, r0y, x, y, mo0, mo1, ds, sink);
+        } else {
+          FixedSink<Tile> sink{TileSink<Tile>(tile, 0, 0, win, L0, L1), a.acc_scale, a.narrow != 0};
+          fits = deposit_move<ORDER, false>(COMP, cur.q, r0x, r0y, x, y, mo0, mo1, ds, sink) ||
+                 deposit_general<ORDER, COMP, Tile>(cur.q, r0x, r0y, x, y, mo0, mo1, ds,
+                                                    FixedSink<Tile>{TileSink<Tile>(tile, 0, 0, win, L0, L1), a.acc_scale,
+                                                                    a.narrow != 0});
+        }
+        if (!fits) overflow = true;
+        lower(amn0, x); lower(amn0, r0x); lower(amn1, y); lower(amn1, r0y);
+        upper(amx0, x); upper(amx0, r0x); upper(amx1, y); upper(amx1, r0y);
+        // next push gathers at (R2 - h v) + h v
+        const double nx = (x + (-w0)) + w0, ny = (y + (-w1)) + w1;
+        lower(bmn0, nx); lower(bmn1, ny); upper(bmx0, nx); upper(bmx1, ny);
+      }
     }
   }
   tile.template flush<SMEM>(win, L0, L1);
   if (overflow) set_err(ws, kErrCrossings);
-  block_bbox(amn0, amn1, amx0, amx1, ws->bball, sh.sb);
-  block_bbox(bmn0, bmn1, bmx0, bmx1, ws->bb[1 - ws->cur], sh.sb);
+  const long long boxes[8] = {dbl_ord(amn0), dbl_ord(amn1), ~dbl_ord(amx0), ~dbl_ord(amx1),
+                              dbl_ord(bmn0), dbl_ord(bmn1), ~dbl_ord(bmx0), ~dbl_ord(bmx1)};
+  merge_boxes(boxes, ws, sh.sb);
   if (SMEM) {
     if (tile.ti1 >= 0) {
       atomicMin(&tb[0], tile.ti0); atomicMin(&tb[1], tile.tj0);
@@ -213,29 +236,37 @@ __device__ __forceinline__ void push_body(const PushArgs &a, long long beg, long
 }
 
 // The single-member push: warp tiles in dynamic shared memory, the window
-// accumulator in global memory, three CTAs per SM.  The push is bound by the
-// latency of dependent FP64 chains; a CTA copy of the accumulator in shared
-// memory held the SM to two CTAs and cost more to zero and flush than the
-// global adds it saved (4e6-particle TSC bunch, 8192 x 1024 mesh: 0.55 ->
-// 0.44 ms per push).  Integer sums: the result does not depend on where
-// they are added.
-template <int ORDER>
-__global__ void __launch_bounds__(256, 3) k_push(PushArgs a) {
+// accumulator in global memory.  It is bound by the latency of dependent FP64
+// chains (divisions and square roots among them) and, with 1640 instructions
+// per particle, by the instruction cache: the component is a template
+// parameter, the crossing list a call, the reciprocals kernel parameters, and
+// the next particle is read a round ahead.  Two CTAs per SM: at three, 80
+// registers a thread spill 360 bytes (8192 x 1024 mesh, 4e6 TSC particles, per
+// step: 795 us at three without the read ahead, 813 with it, 758 at two; 975
+// before).  A CTA copy of the accumulator in shared memory cost more to zero and
+// flush than the global adds it saved.  Integer sums: the result does not
+// depend on where they are added.  The last CTA swaps the box sets, derives the
+// deposit bounds and, when nothing moves the particles or the window before the
+// next push, sets up its gather patches.
+template <int ORDER, int COMP>
+__global__ void __launch_bounds__(kPushThreads, kPushCtas) k_push(PushArgs a) {
   extern __shared__ unsigned long long sacc[];
   __shared__ PushShared sh;
-  const long long per = (a.n + gridDim.x - 1) / gridDim.x;
-  const long long beg = (long long)blockIdx.x * per;
-  const long long end = beg + per < a.n ? beg + per : a.n;
-  push_body<ORDER, false>(a, beg, end, sh, sacc);
+  push_body<ORDER, COMP, false>(a, BunchWork{a.n, push_ctl(a.ws)}, sh, sacc);
+  if (last_cta(a.ws, sh) && threadIdx.x == 0) {
+    a.ws->cur = 1 - a.ws->cur;
+    global_bounds_body(a.ws, a.ds.h0, a.ds.h1);
+    if (a.prep_next) push_prep_body(a.ws, a.ds.h0, a.ds.h1, a.em0, a.em2, a.cm0, true);
+  }
 }
 
 // One push over a batch of members: the members' particles form one index
 // range (ppre: first particle of each member, m + 1 entries) that is cut into
 // equal contiguous shares, one per CTA; a CTA runs the push of every member
 // its share overlaps, with that member's shape order and accumulator.
-template <int ORDER>
-__global__ void __launch_bounds__(256, 2) k_push_batch(const PushArgs *args, const unsigned char *smem_ok,
-                                                       const long long *ppre, int m, long long per) {
+template <int ORDER, int COMP>
+__global__ void __launch_bounds__(kPushThreads, 2) k_push_batch(const PushArgs *args, const unsigned char *smem_ok,
+                                                                const long long *ppre, int m, long long per) {
   extern __shared__ unsigned long long sacc[];
   __shared__ PushShared sh;
   __shared__ PushArgs sa;
@@ -249,39 +280,22 @@ __global__ void __launch_bounds__(256, 2) k_push_batch(const PushArgs *args, con
     __syncthreads();
     if (threadIdx.x == 0) sa = args[mm];
     __syncthreads();
-    if (smem_ok[mm]) push_body<ORDER, true>(sa, lb, le, sh, sacc);
-    else push_body<ORDER, false>(sa, lb, le, sh, sacc);
+    if (smem_ok[mm]) push_body<ORDER, COMP, true>(sa, ShareWork{lb, le}, sh, sacc);
+    else push_body<ORDER, COMP, false>(sa, ShareWork{lb, le}, sh, sacc);
   }
 }
 
 // Per-member bookkeeping of a batched push, one thread per member.
 __global__ void k_push_prep_batch(const PrepArgs *p, int m) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < m) push_prep_body(p[k].ws, p[k].h0, p[k].h1, p[k].em0, p[k].em2, p[k].cm0);
+  if (k < m) push_prep_body(p[k].ws, p[k].h0, p[k].h1, p[k].em0, p[k].em2, p[k].cm0, false);
 }
 __global__ void k_push_post_batch(const PrepArgs *p, int m) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < m) p[k].ws->cur = 1 - p[k].ws->cur;
-}
-
-// After the last push of a step: the deposit's particle bounds relative to
-// the window (PartBunch::getLocalPDomainInclOld -> setGlobalBounds).
-__device__ __forceinline__ void global_bounds_body(WinState *ws, double h0, double h1) {
-  const double mn0 = ord_dbl(ws->bball[0]), mn1 = ord_dbl(ws->bball[1]);
-  const double mx0 = ord_dbl(ws->bball[2]), mx1 = ord_dbl(ws->bball[3]);
-  if (!(mn0 <= mx0)) { ws->gb[0] = 0; ws->gb[1] = -1; ws->gb[2] = 0; ws->gb[3] = -1; return; }
-  ws->gb[0] = (int)floor((mn0 - ws->mo0) / h0);
-  ws->gb[1] = (int)floor((mx0 - ws->mo0) / h0);
-  ws->gb[2] = (int)floor((mn1 - ws->mo1) / h1);
-  ws->gb[3] = (int)floor((mx1 - ws->mo1) / h1);
-}
-
-__global__ void k_global_bounds(WinState *ws, double h0, double h1) {
-  if (threadIdx.x == 0) global_bounds_body(ws, h0, h1);
-}
-__global__ void k_global_bounds_batch(const PrepArgs *p, int m) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < m) global_bounds_body(p[k].ws, p[k].h0, p[k].h1);
+  if (k < m) {
+    p[k].ws->cur = 1 - p[k].ws->cur;
+    global_bounds_body(p[k].ws, p[k].h0, p[k].h1);
+  }
 }
 
 // Stand-alone drift (PartBunch::drift_particles, PartBunch.cpp:179-187).
@@ -318,6 +332,7 @@ __global__ void k_deposit(int comp, const double *ox, const double *oy, const do
                           double h0, double h1, double dt, int i0, int j0, int ni, int nj,
                           unsigned long long *acc, double scale, int *err) {
   // err[0]: crossing overflow; err[1]: a non-zero contribution fell outside the patch
+  const DepositScale ds = deposit_scale<ORDER>(h0, h1, dt);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     bool dropped = false;
@@ -328,7 +343,7 @@ __global__ void k_deposit(int comp, const double *ox, const double *oy, const do
       if (!in && iv != 0) dropped = true;
       warp_add(acc, in ? b * ni + a : -1, iv);
     };
-    if (!deposit_particle<ORDER>(comp, q[i], ox[i], oy[i], x[i], y[i], org0, org1, h0, h1, h0, h1, dt, sink))
+    if (!deposit_particle<ORDER>(comp, q[i], ox[i], oy[i], x[i], y[i], org0, org1, ds, sink))
       atomicExch(&err[0], kErrCrossings);
     if (dropped) atomicExch(&err[1], 1);
   }
@@ -358,8 +373,13 @@ PrepArgs prep_args(WinState *ws, double h0, double h1, int order) {
 }
 
 void launch_push_prep(WinState *ws, double h0, double h1, int order, cudaStream_t s) {
-  const PrepArgs p = prep_args(ws, h0, h1, order);
-  k_push_prep<<<1, 32, 0, s>>>(ws, h0, h1, p.em0, p.em2, p.cm0);
+  k_push_prep<<<1, 32, 0, s>>>(prep_args(ws, h0, h1, order));
+}
+
+void set_push_consts(PushArgs &a, int order, double h0, double h1, double dt) {
+  a.ds = order == 0 ? deposit_scale<0>(h0, h1, dt) : deposit_scale<1>(h0, h1, dt);
+  const PrepArgs p = prep_args(a.ws, h0, h1, order);
+  a.em0 = p.em0; a.em2 = p.em2; a.cm0 = p.cm0;
 }
 
 size_t push_tile_bytes(int order) {
@@ -374,7 +394,7 @@ long long push_batch_smem_limit() {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, k_push_batch<1>);
+    cudaFuncGetAttributes(&fa, k_push_batch<1, 0>);
     lim = (long long)v - (long long)fa.sharedSizeBytes;
     // keep two CTAs per SM: half the SM's shared memory less the static part
     // and the 1 KB the runtime reserves per CTA
@@ -382,13 +402,21 @@ long long push_batch_smem_limit() {
     cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     const long long two = (long long)per_sm / 2 - (long long)fa.sharedSizeBytes - 1024;
     if (two > 0 && two < lim) lim = two;
-    if (cudaFuncSetAttribute(k_push_batch<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) != cudaSuccess ||
-        cudaFuncSetAttribute(k_push_batch<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) != cudaSuccess ||
-        cudaFuncSetAttribute(k_push_batch<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) != cudaSuccess)
-      lim = 0;
+    auto opt_in = [&](auto *kernel) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) != cudaSuccess) lim = 0;
+    };
+    opt_in(k_push_batch<0, 0>); opt_in(k_push_batch<0, 1>);
+    opt_in(k_push_batch<1, 0>); opt_in(k_push_batch<1, 1>);
+    opt_in(k_push_batch<2, 0>); opt_in(k_push_batch<2, 1>);
     cudaGetLastError();
   }
   return lim;
+}
+
+template <int ORDER>
+static void push_batch_order(const PushArgs *args, const PushGroup &G, int ctas, long long per, cudaStream_t s) {
+  if (G.jcomp == 0) k_push_batch<ORDER, 0><<<ctas, kPushThreads, G.smem, s>>>(args, G.smem_ok, G.ppre, G.m, per);
+  else k_push_batch<ORDER, 1><<<ctas, kPushThreads, G.smem, s>>>(args, G.smem_ok, G.ppre, G.m, per);
 }
 
 void launch_push_batch(const PushGroup *groups, int ngroups, int m, int grid, const PrepArgs *prep, cudaStream_t s,
@@ -401,39 +429,34 @@ void launch_push_batch(const PushGroup *groups, int ngroups, int m, int grid, co
     const int ctas = (int)((long long)grid * G.total / (G.all > 0 ? G.all : G.total)) + 1;
     const long long per = (G.total + ctas - 1) / ctas;
     const PushArgs *args = static_cast<const PushArgs *>(G.args);
-    if (G.order == 0) k_push_batch<0><<<ctas, 256, G.smem, s>>>(args, G.smem_ok, G.ppre, G.m, per);
-    else if (G.order == 1) k_push_batch<1><<<ctas, 256, G.smem, s>>>(args, G.smem_ok, G.ppre, G.m, per);
-    else k_push_batch<2><<<ctas, 256, G.smem, s>>>(args, G.smem_ok, G.ppre, G.m, per);
+    if (G.order == 0) push_batch_order<0>(args, G, ctas, per, s);
+    else if (G.order == 1) push_batch_order<1>(args, G, ctas, per, s);
+    else push_batch_order<2>(args, G, ctas, per, s);
   }
-  if (parts & 2) {
-    k_push_post_batch<<<tb, 128, 0, s>>>(prep, m);
-    k_global_bounds_batch<<<tb, 128, 0, s>>>(prep, m);
-  }
+  if (parts & 2) k_push_post_batch<<<tb, 128, 0, s>>>(prep, m);
 }
 
 // Dynamic shared memory of the single-member push: its warp tiles (48-56 KB,
 // above the 48 KB a launch gets without opting in).
 template <int ORDER>
-static size_t push_smem() {
+static void push_order(const PushArgs &a, int grid, cudaStream_t s) {
   static int set = 0;
-  const size_t tiles = (size_t)TileFor<ORDER>::T::kSize * 256 * sizeof(unsigned long long);
+  const size_t tiles = (size_t)TileFor<ORDER>::T::kSize * kPushThreads * sizeof(unsigned long long);
   if (!set) {
-    cudaFuncSetAttribute(k_push<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiles);
+    cudaFuncSetAttribute(k_push<ORDER, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiles);
+    cudaFuncSetAttribute(k_push<ORDER, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiles);
     cudaGetLastError();
     set = 1;
   }
-  return tiles;
+  const int g = push_ctas(a.n, grid);
+  if (a.jcomp == 0) k_push<ORDER, 0><<<g, kPushThreads, tiles, s>>>(a);
+  else k_push<ORDER, 1><<<g, kPushThreads, tiles, s>>>(a);
 }
 
 void launch_push(const PushArgs &a, int order, int grid, cudaStream_t s) {
-  if (order == 0) k_push<0><<<grid, 256, push_smem<0>(), s>>>(a);
-  else if (order == 1) k_push<1><<<grid, 256, push_smem<1>(), s>>>(a);
-  else k_push<2><<<grid, 256, push_smem<2>(), s>>>(a);
-  k_push_post<<<1, 32, 0, s>>>(a.ws);
-}
-
-void launch_global_bounds(WinState *ws, double h0, double h1, cudaStream_t s) {
-  k_global_bounds<<<1, 32, 0, s>>>(ws, h0, h1);
+  if (order == 0) push_order<0>(a, grid, s);
+  else if (order == 1) push_order<1>(a, grid, s);
+  else push_order<2>(a, grid, s);
 }
 
 void launch_drift(double *x, double *y, const double *px, const double *py, long long n, double full,

@@ -213,57 +213,12 @@ struct Boxes32 {
     amx0 = max(amx0, max(r0, m.ni)); amx1 = max(amx1, max(r1, m.nj));
     bmn0 = min(bmn0, m.ni); bmn1 = min(bmn1, m.nj); bmx0 = max(bmx0, m.ni); bmx1 = max(bmx1, m.nj);
   }
-  __device__ __forceinline__ static double c(int v, bool lo) {
-    return lo ? (v == INT_MAX ? INFINITY : v + 0.5) : (v == INT_MIN ? -INFINITY : v + 0.5);
-  }
+  // cells as cell + 0.5, ordered; nothing added: +-infinity
+  __device__ __forceinline__ static long long lo(int v) { return dbl_ord(v == INT_MAX ? INFINITY : v + 0.5); }
+  __device__ __forceinline__ static long long hi(int v) { return ~dbl_ord(v == INT_MIN ? -INFINITY : v + 0.5); }
   __device__ __forceinline__ void store(WinState *ws, PushShared &sh) {
-    block_bbox(c(amn0, true), c(amn1, true), c(amx0, false), c(amx1, false), ws->bball, sh.sb);
-    block_bbox(c(bmn0, true), c(bmn1, true), c(bmx0, false), c(bmx1, false), ws->bb[1 - ws->cur], sh.sb);
-  }
-};
-
-// Adds one particle's deposit to its warp's tile.  The whole stencil box is
-// checked against the tile once; inside it every entry is a load, an add and a
-// store at a compile-time offset from one address.  Boxes that do not fit go to
-// the tile or the window accumulator entry by entry.
-template <class Tile>
-struct TileSink {
-  unsigned long long *tile;  // this lane's tile
-  int bi, bj;                // its first window cell
-  int wi, wj;                // the particle's old cell (window cells)
-  unsigned long long *acc;
-  int L0, L1;
-  unsigned long long *p;
-  int j0;
-  bool in;
-  __device__ __forceinline__ TileSink(const Tile &t, int wi_, int wj_, unsigned long long *acc_, int L0_, int L1_)
-      : tile(t.tile), bi(t.bi - Tile::kOX), bj(t.bj - Tile::kOY), wi(wi_), wj(wj_), acc(acc_), L0(L0_), L1(L1_) {}
-  template <int NX, int NY>
-  __device__ __forceinline__ void box(int i, int j) {
-    const int a = wi + i - bi, b = wj + j - bj;
-    // a box larger than the tile (the cubic shape's general form) never fits
-    in = NX <= Tile::kTW && NY <= Tile::kTH && a >= 0 && a <= Tile::kTW - NX && b >= 0 && b <= Tile::kTH - NY;
-    p = tile + (b * Tile::kTW + a) * kPushThreads;
-    j0 = j;
-  }
-  template <int N>
-  __device__ __forceinline__ void row(int i, int j, const long long (&v)[N]) {
-    if (in) {
-#pragma unroll
-      for (int c = 0; c < N; ++c) p[((j - j0) * Tile::kTW + c) * kPushThreads] += (unsigned long long)v[c];
-    } else {
-#pragma unroll
-      for (int c = 0; c < N; ++c)
-        if (v[c] != 0) put(tile, wi + i + c - bi, wj + j - bj, acc, wi + i + c, wj + j, L0, L1, v[c]);
-    }
-  }
-  // one entry at (a, b) of the tile, window cell (i, j)
-  static __device__ __forceinline__ void put(unsigned long long *tile, int a, int b, unsigned long long *acc, int i, int j,
-                                          int L0, int L1, long long v) {
-    if ((unsigned)a < (unsigned)Tile::kTW && (unsigned)b < (unsigned)Tile::kTH)
-      tile[(b * Tile::kTW + a) * kPushThreads] += (unsigned long long)v;
-    else if (i >= 0 && j >= 0 && i < L0 && j < L1)
-      atomicAdd(&acc[j * L0 + i], (unsigned long long)v);
+    const long long v[8] = {lo(amn0), lo(amn1), hi(amx0), hi(amx1), lo(bmn0), lo(bmn1), hi(bmx0), hi(bmx1)};
+    merge_boxes(v, ws, sh.sb);
   }
 };
 
@@ -284,13 +239,14 @@ __device__ __forceinline__ void push32_range(const Push32Args &a, const Work &wo
   tile.init(sm, L0, L1);
   Boxes32 box;
   bool overflow = false;
+  const int lane = threadIdx.x & 31;
   long long n0, end, step;
   for (int k = 0; work.run(k, n0, end, step); ++k) {
     // each lane's next particle is read while the current one moves
     In32 next{};
-    if (n0 + threadIdx.x < end) next = load32(a.b, n0 + threadIdx.x);
+    if (n0 + lane < end) next = load32(a.b, n0 + lane);
     for (; n0 < end; n0 += step) {  // the same rounds for every lane of the warp
-      const long long n = n0 + threadIdx.x;
+      const long long n = n0 + lane;
       const In32 cur = next;
       if (n + step < end) next = load32(a.b, n + step);
       Move32 m;
@@ -322,28 +278,6 @@ __device__ __forceinline__ void push32_range(const Push32Args &a, const Work &wo
   tile.template flush<false>(a.acc, L0, L1);
   if (overflow) set_err(ws, kErrCrossings);
   box.store(ws, sh);
-  __syncthreads();
-}
-
-// Gather-patch set-up and the window-fit check from the box of the next
-// push's gather positions (cells of the static mesh).  defer: a bunch that does
-// not fit is reported by the next push, not at once (PushCtl).
-__device__ __forceinline__ void prep32_body(WinState *ws, int reach, bool defer) {
-  const int c = ws->cur;
-  const double mn0 = ord_dbl(ws->bb[c][0]), mn1 = ord_dbl(ws->bb[c][1]);
-  const double mx0 = ord_dbl(ws->bb[c][2]), mx1 = ord_dbl(ws->bb[c][3]);
-  int nofit = 0;
-  if (mn0 <= mx0) {
-    const int lp[4] = {(int)floor(mn0) - ws->P0, (int)floor(mx0) - ws->P0, (int)floor(mn1) - ws->P1,
-                       (int)floor(mx1) - ws->P1};
-    for (int k = 0; k < 4; ++k) ws->lp[k] = lp[k];
-    // every gather tap lies within [lp - reach, lp + reach]
-    nofit = lp[0] - reach < -1 || lp[1] + reach > ws->L0 || lp[2] - reach < -1 || lp[3] + reach > ws->L1;
-    if (nofit && !defer) set_err(ws, kErrWindowFit);
-  }
-  push_ctl(ws)->nofit = defer ? nofit : 0;
-  bbox_reset(ws->bb[1 - c]);
-  bbox_reset(ws->bball);
 }
 
 // Deposit bounds in window cells (PartBunch::getLocalPDomainInclOld).
@@ -364,7 +298,7 @@ template <int ORDER, int COMP>
 __global__ void __launch_bounds__(kPushThreads, Push32Occ<ORDER>::kCtas) k_push32(Push32Args a) {
   extern __shared__ unsigned long long sacc[];
   __shared__ PushShared sh;
-  push32_range<ORDER, COMP>(a, BunchWork{a.b.n}, sh, sacc);
+  push32_range<ORDER, COMP>(a, BunchWork{a.b.n, push_ctl(a.ws)}, sh, sacc);
   // the last CTA swaps the box sets (the push filled the other one), derives
   // the deposit bounds and, when nothing moves the particles or the window
   // before the next push, sets up its gather patch

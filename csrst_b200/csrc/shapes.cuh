@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "sinkbox.cuh"
 
 namespace csrst {
 
@@ -38,32 +39,28 @@ template <int ORDER, class F, class S>
 __device__ __forceinline__ S gather_edge(const F &f, S pp0, S pp1, int comp) {
   const S one = S(1), half = S(0.5), zero = S(0);
   if (ORDER == 0) {
-    long l0 = (long)floor(pp0 + (comp == 0 ? half : zero));
-    long l1 = (long)floor(pp1 + (comp == 1 ? half : zero));
-    if (comp == 0) l0 -= 1; else l1 -= 1;
-    S g0 = (S)l0, g1 = (S)l1;
+    // the floors stay in S: their integer values are exact there
+    S g0 = floor(pp0 + (comp == 0 ? half : zero)), g1 = floor(pp1 + (comp == 1 ? half : zero));
+    if (comp == 0) g0 -= one; else g1 -= one;
+    const int I = (int)g0, J = (int)g1;
     if (comp == 0) g0 += half; else g1 += half;
     const S d0 = pp0 - g0, d1 = pp1 - g1;
-    const int I = (int)l0, J = (int)l1;
     return ((one - d1) * ((one - d0) * f(I, J) + d0 * f(I + 1, J)) +
             d1 * ((one - d0) * f(I, J + 1) + d0 * f(I + 1, J + 1)));
   } else if (ORDER == 1) {
-    long l0 = (long)floor(pp0 + (comp == 0 ? zero : half));
-    long l1 = (long)floor(pp1 + (comp == 1 ? zero : half));
-    S g0 = (S)l0, g1 = (S)l1;
+    S g0 = floor(pp0 + (comp == 0 ? zero : half)), g1 = floor(pp1 + (comp == 1 ? zero : half));
+    const int I = (int)g0, J = (int)g1;
     if (comp == 0) g0 += half; else g1 += half;
     const S d0 = pp0 - g0, d1 = pp1 - g1;
     const S bx = S(0.75) - d0 * d0, cx = half * (half + d0) * (half + d0), ax = one - (bx + cx);
     const S by = S(0.75) - d1 * d1, cy = half * (half + d1) * (half + d1), ay = one - (by + cy);
-    const int I = (int)l0, J = (int)l1;
     return (ay * (ax * f(I - 1, J - 1) + bx * f(I, J - 1) + cx * f(I + 1, J - 1)) +
             by * (ax * f(I - 1, J) + bx * f(I, J) + cx * f(I + 1, J)) +
             cy * (ax * f(I - 1, J + 1) + bx * f(I, J + 1) + cx * f(I + 1, J + 1)));
   } else {
-    long l0 = (long)floor(pp0 + (comp == 0 ? half : zero));
-    long l1 = (long)floor(pp1 + (comp == 1 ? half : zero));
-    if (comp == 0) l0 -= 1; else l1 -= 1;
-    S g0 = (S)l0, g1 = (S)l1;
+    S g0 = floor(pp0 + (comp == 0 ? half : zero)), g1 = floor(pp1 + (comp == 1 ? half : zero));
+    if (comp == 0) g0 -= one; else g1 -= one;
+    const int I = (int)g0, J = (int)g1;
     if (comp == 0) g0 += half; else g1 += half;
     const S d0 = pp0 - g0, d1 = pp1 - g1;
     const S q0 = d0 * d0, q1 = d1 * d1;
@@ -72,7 +69,6 @@ __device__ __forceinline__ S gather_edge(const F &f, S pp0, S pp1, int comp) {
     const S ax = one - (bx + cx + ex);
     const S by = t23 - q1 * (one - half * d1), cy = t23 - half * (one - d1) * (one - q1), ey = t16 * q1 * d1;
     const S ay = one - (by + cy + ey);
-    const int I = (int)l0, J = (int)l1;
     // The last term reads (I+1, J+2), as the reference does (ScatterGatherImpl.hh:467).
     return (ay * (ax * f(I - 1, J - 1) + bx * f(I, J - 1) + cx * f(I + 1, J - 1) + ex * f(I + 2, J - 1)) +
             by * (ax * f(I - 1, J) + bx * f(I, J) + cx * f(I + 1, J) + ex * f(I + 2, J)) +
@@ -86,30 +82,30 @@ template <int ORDER, class F, class S>
 __device__ __forceinline__ S gather_cell(const F &f, S pp0, S pp1) {
   const S one = S(1), half = S(0.5);
   if (ORDER == 0) {
-    const long l0 = (long)floor(pp0 - half), l1 = (long)floor(pp1 - half);
-    const S d0 = pp0 - ((S)l0 + half), d1 = pp1 - ((S)l1 + half);
+    const S l0 = floor(pp0 - half), l1 = floor(pp1 - half);
+    const S d0 = pp0 - (l0 + half), d1 = pp1 - (l1 + half);
     const int I = (int)l0, J = (int)l1;
     return ((one - d1) * ((one - d0) * f(I, J) + d0 * f(I + 1, J)) +
             d1 * ((one - d0) * f(I, J + 1) + d0 * f(I + 1, J + 1)));
   } else if (ORDER == 1) {
-    const long l0 = (long)floor(pp0), l1 = (long)floor(pp1);
-    const S d0 = pp0 - ((S)l0 + half), d1 = pp1 - ((S)l1 + half);
+    const S l0 = floor(pp0), l1 = floor(pp1);
+    const S d0 = pp0 - (l0 + half), d1 = pp1 - (l1 + half);
+    const int I = (int)l0, J = (int)l1;
     const S bx = S(0.75) - d0 * d0, cx = half * (half + d0) * (half + d0), ax = one - (bx + cx);
     const S by = S(0.75) - d1 * d1, cy = half * (half + d1) * (half + d1), ay = one - (by + cy);
-    const int I = (int)l0, J = (int)l1;
     return (ay * (ax * f(I - 1, J - 1) + bx * f(I, J - 1) + cx * f(I + 1, J - 1)) +
             by * (ax * f(I - 1, J) + bx * f(I, J) + cx * f(I + 1, J)) +
             cy * (ax * f(I - 1, J + 1) + bx * f(I, J + 1) + cx * f(I + 1, J + 1)));
   } else {
-    const long l0 = (long)floor(pp0 - half), l1 = (long)floor(pp1 - half);
-    const S d0 = pp0 - ((S)l0 + half), d1 = pp1 - ((S)l1 + half);
+    const S l0 = floor(pp0 - half), l1 = floor(pp1 - half);
+    const S d0 = pp0 - (l0 + half), d1 = pp1 - (l1 + half);
+    const int I = (int)l0, J = (int)l1;
     const S q0 = d0 * d0, q1 = d1 * d1;
     const S t23 = S(2.0 / 3.0), t16 = S(1.0 / 6.0);
     const S bx = t23 - q0 * (one - half * d0), cx = t23 - half * (one - d0) * (one - q0), ex = t16 * q0 * d0;
     const S ax = one - (bx + cx + ex);
     const S by = t23 - q1 * (one - half * d1), cy = t23 - half * (one - d1) * (one - q1), ey = t16 * q1 * d1;
     const S ay = one - (by + cy + ey);
-    const int I = (int)l0, J = (int)l1;
     return (ay * (ax * f(I - 1, J - 1) + bx * f(I, J - 1) + cx * f(I + 1, J - 1) + ex * f(I + 2, J - 1)) +
             by * (ax * f(I - 1, J) + bx * f(I, J) + cx * f(I + 1, J) + ex * f(I + 2, J)) +
             cy * (ax * f(I - 1, J + 1) + bx * f(I, J + 1) + cx * f(I + 1, J + 1) + ex * f(I + 2, J + 1)) +
@@ -184,13 +180,29 @@ __device__ __forceinline__ int border_crossings(Cross *xs, double o0, double o1,
   return num;
 }
 
+// Constants of a deposit on a mesh of spacing (h0, h1) with time step dt, as
+// the reference forms them; host code computes the same bits, so that a push
+// reads them as kernel parameters.
+struct DepositScale {
+  double h0, h1, ood0, ood1, oodt0, oodt1;
+};
+template <int ORDER>
+__host__ __device__ inline DepositScale deposit_scale(double h0, double h1, double dt) {
+  DepositScale s{h0, h1, 1.0 / h0, 1.0 / h1, 0.0, 0.0};
+  if (ORDER == 0) { s.oodt0 = 1.0 / (h1 * dt); s.oodt1 = 1.0 / (h0 * dt); }
+  else { s.oodt0 = s.ood0 / dt; s.oodt1 = s.ood1 / dt; }
+  return s;
+}
+
 // Current of one straight segment a -> b (subSteps relative to the mesh
 // origin) of a particle whose whole push covers the displacement dl (cells)
-// and distance cov; sink(i, j, value) receives every contribution.
+// and distance cov; sink(i, j, value) receives every contribution, the box
+// they lie in announced first (open_box).
 template <int ORDER, class Sink>
 __device__ __forceinline__ void deposit_segment(int comp, double q, double a0, double a1, double b0, double b1,
-                                                double ood0, double ood1, double oodt0, double oodt1,
-                                                double dl0, double dl1, double cov, Sink &sink) {
+                                                const DepositScale &ds, double dl0, double dl1, double cov,
+                                                Sink &sink) {
+  const double ood0 = ds.ood0, ood1 = ds.ood1, oodt0 = ds.oodt0, oodt1 = ds.oodt1;
   const double xi0 = a0 * ood0, xi1 = a1 * ood1;
   const double xf0 = b0 * ood0, xf1 = b1 * ood1;
   if (ORDER == 0) {
@@ -198,10 +210,12 @@ __device__ __forceinline__ void deposit_segment(int comp, double q, double a0, d
     const double c0 = (xi0 + xf0) * 0.5, c1 = (xi1 + xf1) * 0.5;
     const int I = (int)floor(c0), J = (int)floor(c1);
     if (comp == 0) {
+      open_box<1, 2>(sink, I, J, 0);
       const double D0 = q * (xf0 - xi0) * oodt0;
       sink(I, J, D0 * (J + 1 - c1));
       sink(I, J + 1, D0 * (c1 - J));
     } else {
+      open_box<2, 1>(sink, I, J, 0);
       const double D1 = q * (xf1 - xi1) * oodt1;
       sink(I, J, D1 * (I + 1 - c0));
       sink(I + 1, J, D1 * (c0 - I));
@@ -234,6 +248,8 @@ __device__ __forceinline__ void deposit_segment(int comp, double q, double a0, d
     A2[2] = half * (half - b_cr) * (half - b_cr) * tau;
     B2[2] = (half - b_cr) * d_cr * tp2;
     C2[2] = half * d_cr * d_cr * tp3;
+    if (comp == 0) open_box<2, 3>(sink, I - 1, J - 1, 0);
+    else open_box<3, 2>(sink, I - 1, J - 1, 0);
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
       const double sm = A2[t] + B2[t] + C2[t];
@@ -286,6 +302,8 @@ __device__ __forceinline__ void deposit_segment(int comp, double q, double a0, d
     tB[3] = b * b * de * half * tp2;
     tC[3] = -b * de2 * half * tp3;
     tD[3] = de3 * onesixth * tp4;
+    if (comp == 0) open_box<3, 4>(sink, I - 1, J - 1, 0);
+    else open_box<4, 3>(sink, I - 1, J - 1, 0);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
 #pragma unroll
@@ -318,9 +336,9 @@ __device__ __forceinline__ int floor_div(double v, double h, double ooh, double 
 }
 
 template <bool DUAL, class Seg>
-__device__ __forceinline__ bool segments_fast(double o0, double o1, double n0, double n1, double h0, double h1,
+__device__ __forceinline__ bool segments_fast(double o0, double o1, double n0, double n1, const DepositScale &ds,
                                               Seg &&seg) {
-  const double sh = DUAL ? 0.5 : 0.0, ooh0 = 1.0 / h0, ooh1 = 1.0 / h1;
+  const double sh = DUAL ? 0.5 : 0.0, h0 = ds.h0, h1 = ds.h1, ooh0 = ds.ood0, ooh1 = ds.ood1;
   const int Ii = floor_div(o0, h0, ooh0, sh), Ji = floor_div(o1, h1, ooh1, sh);
   const int If = floor_div(n0, h0, ooh0, sh), Jf = floor_div(n1, h1, ooh1, sh);
   if (abs(If - Ii) > 1 || abs(Jf - Ji) > 1) return false;
@@ -361,39 +379,37 @@ __device__ __forceinline__ bool segments_fast(double o0, double o1, double n0, d
 
 // Calls sink(i, j, value) for every current contribution of one particle
 // moving old -> new (absolute positions; the mesh origin is org; indices are
-// mesh cells).  Returns false on a crossing overflow.  (h0, h1) is the
-// spacing of the coordinates given; (jh0, jh1) the physical spacing that
-// scales the current.  The FP64 path passes physical positions with
-// jh = h; FP32 mode passes positions in cells (h = 1).  Ratios of lengths
-// along one straight move do not depend on the units, so both give the
-// same current up to rounding.
-template <int ORDER, class Sink>
-__device__ __forceinline__ bool deposit_particle(int comp, double q, double ao0, double ao1, double an0,
-                                                 double an1, double org0, double org1, double h0, double h1,
-                                                 double jh0, double jh1, double dt, Sink &&sink) {
+// mesh cells).  GENERAL: any number of crossings, false on an overflow; else
+// the moves segments_fast takes, false for others (nothing is emitted then).
+template <int ORDER, bool GENERAL, class Sink>
+__device__ __forceinline__ bool deposit_move(int comp, double q, double ao0, double ao1, double an0, double an1,
+                                             double org0, double org1, const DepositScale &ds, Sink &&sink) {
   // crossings are taken relative to the mesh origin (utils.hh:435-436)
   const double o0 = ao0 - org0, o1 = ao1 - org1, n0 = an0 - org0, n1 = an1 - org1;
-  const double ood0 = 1.0 / h0, ood1 = 1.0 / h1;
-  double oodt0, oodt1, dl0 = 0.0, dl1 = 0.0, cov = 0.0;
-  if (ORDER == 0) {
-    oodt0 = 1.0 / (jh1 * dt); oodt1 = 1.0 / (jh0 * dt);
-  } else {
+  double dl0 = 0.0, dl1 = 0.0, cov = 0.0;
+  if (ORDER > 0) {
     // the full displacement uses the absolute positions (R - oldR)
     const double Dx0 = an0 - ao0, Dx1 = an1 - ao1;
     cov = sqrt(Dx0 * Dx0 + Dx1 * Dx1);
     if (cov == 0.0) return true;  // a particle that does not move carries no current
-    oodt0 = (1.0 / jh0) / dt; oodt1 = (1.0 / jh1) / dt;
-    dl0 = Dx0 * ood0; dl1 = Dx1 * ood1;
+    dl0 = Dx0 * ds.ood0; dl1 = Dx1 * ds.ood1;
   }
   auto seg = [&](double a0, double a1, double b0, double b1) {
-    deposit_segment<ORDER>(comp, q, a0, a1, b0, b1, ood0, ood1, oodt0, oodt1, dl0, dl1, cov, sink);
+    deposit_segment<ORDER>(comp, q, a0, a1, b0, b1, ds, dl0, dl1, cov, sink);
   };
-  if (segments_fast<ORDER == 1>(o0, o1, n0, n1, h0, h1, seg)) return true;
+  if constexpr (!GENERAL) return segments_fast<ORDER == 1>(o0, o1, n0, n1, ds, seg);
   Cross xs[kMaxCross];
-  const int n = border_crossings<ORDER == 1>(xs, o0, o1, n0, n1, h0, h1);
+  const int n = border_crossings<ORDER == 1>(xs, o0, o1, n0, n1, ds.h0, ds.h1);
   if (n < 0) return false;
   for (int k = 0; k + 1 < n; ++k) seg(xs[k].s0, xs[k].s1, xs[k + 1].s0, xs[k + 1].s1);
   return true;
+}
+template <int ORDER, class Sink>
+__device__ __forceinline__ bool deposit_particle(int comp, double q, double ao0, double ao1, double an0,
+                                                 double an1, double org0, double org1, const DepositScale &ds,
+                                                 Sink &&sink) {
+  return deposit_move<ORDER, false>(comp, q, ao0, ao1, an0, an1, org0, org1, ds, sink) ||
+         deposit_move<ORDER, true>(comp, q, ao0, ao1, an0, an1, org0, org1, ds, sink);
 }
 
 // Warp-aggregated fixed-point add: lanes that target the same cell combine

@@ -1,7 +1,7 @@
 """How a push shares its bunch out over the grid (csrc/pushwork.cuh): every
 particle is moved and deposited exactly once for bunches of one particle, of
-one CTA round and around it, of two rounds per CTA, and large enough for the rim
-of the bunch to be dealt out round by round (16 rounds per CTA).  The check is
+one CTA round and around it, of two rounds per CTA, and large enough for a part
+of the bunch to be handed out by a counter (8 rounds per CTA).  The check is
 exact: the window current after a push is, integer for integer, the stand-alone
 deposit of the moves the push made."""
 import numpy as np
@@ -44,4 +44,27 @@ def test_fp32_push_moves_every_particle_once(gpu_lib, order, n):
         assert np.array_equal(s.window_field(4 + comp)[1:L1 + 1, 1:L0 + 1], F.astype(np.float64) * inv)
         s.update_e(comp)
         s.drift(-0.5 * info["dt"])
+    s.close()
+
+
+@pytest.mark.parametrize("order,n", SIZES)
+def test_fp64_push_moves_every_particle_once(gpu_lib, order, n):
+    """The FP64 push rounds each contribution by an FP64 add for bunches of
+    1024 particles or more and by a conversion for smaller ones."""
+    s = loaded(order, n, False)
+    s.step(2)
+    info = s.info()
+    h, dt, scale = (info["hx"], info["hy"]), info["dt"], info["fixed_scale"]
+    q = np.full(n, make_bunch(workload(f"small-{order}")[1])[4][0] * 4000 / n)  # equal charges, any order
+    sf = ShapeFunction(order)
+    for comp in (0, 1):
+        s.push(comp)
+        x, y, _, _ = s.particles()
+        ox, oy = s.old_positions()
+        (_, _, L0, L1), org, _ = s.window()
+        J = sf.getCurrentDensityBase(comp, ox, oy, x, y, q, org, h, dt, 0, 0, L0, L1, scale)
+        assert comp == 1 or np.abs(J).max() > 0
+        assert np.array_equal(s.window_field(4 + comp)[1:L1 + 1, 1:L0 + 1], J)
+        s.update_e(comp)
+        s.drift(-0.5 * dt)
     s.close()
