@@ -395,6 +395,19 @@ void pfree(void *p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }
 
+}  // namespace
+
+cudaError_t csrst::ScratchBuffer::alloc(size_t bytes) {
+  pooled = bytes <= kKeep;
+  return pooled ? palloc(&p, bytes, s) : cudaMalloc(&p, bytes);
+}
+csrst::ScratchBuffer::~ScratchBuffer() {
+  if (pooled) pfree(p, s);
+  else cudaFree(p);
+}
+
+namespace {
+
 void drop_graphs(csrst_handle *h) {
   for (cudaGraphExec_t &g : h->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
@@ -1152,15 +1165,18 @@ int csrst_initial_fields(csrst_handle *h, double tol_first, double tol_rest, int
   in.tol_first = tol_first; in.tol_rest = tol_rest; in.maxit = max_iter;
   // FP32 mode solves in FP64 (the bunch converted, the planes staged) and
   // rounds the fields once
+  ScratchBuffer qbuf(h->s), sbuf(h->s);
   double *qd = nullptr, *stage = nullptr;
   const size_t ps = (size_t)h->pitch * (h->b.Ny + 2);
   if (h->fp32) {
     int pend = 0;
     bunch64(h, &in.x, &in.y, &in.px, &in.py, &pend);
-    CK(cudaMalloc(&qd, (size_t)h->n * sizeof(double)));
+    CK(qbuf.alloc((size_t)h->n * sizeof(double)));
+    qd = static_cast<double *>(qbuf.p);
     launch_f2d(h->b32.q, (int)h->n, qd, (int)h->n, 1, (int)h->n, h->s);
     in.q = qd;
-    CK(cudaMalloc(&stage, 4 * ps * sizeof(double)));
+    CK(sbuf.alloc(4 * ps * sizeof(double)));
+    stage = static_cast<double *>(sbuf.p);
     CK(cudaMemsetAsync(stage, 0, 4 * ps * sizeof(double), h->s));
     in.Ex = plane(stage, h->pitch); in.Ey = plane(stage + ps, h->pitch);
     in.Hx = plane(stage + 2 * ps, h->pitch); in.Hy = plane(stage + 3 * ps, h->pitch);
@@ -1176,10 +1192,7 @@ int csrst_initial_fields(csrst_handle *h, double tol_first, double tol_rest, int
     float *dst[4] = {h->Exf, h->Eyf, h->Hxf, h->Hyf};
     for (int k = 0; k < 4; ++k)
       launch_d2f(stage + k * ps, h->pitch, dst[k], h->pitch32, h->b.Ny + 2, h->b.Nx + 2, h->s);
-    cudaStreamSynchronize(h->s);
   }
-  cudaFree(qd);
-  cudaFree(stage);
   if (rc) return fail(h, rc == kErrCuda ? CSRST_E_CUDA : CSRST_E_ARG, "initial fields: " + msg);
   // resetOutsideDomain, then copyFields + exchangeBoundaries (main.cpp:248, :335-342)
   if (h->fp32) launch_reset_outside(field_args32(h, 0), h->cutidx, h->s);

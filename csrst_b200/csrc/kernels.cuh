@@ -110,6 +110,23 @@ struct PushGroup {
   size_t smem;                      // dynamic shared memory of the group's launch
 };
 
+// One device buffer of a call, freed in the order of its stream.  Up to
+// kKeep bytes come from the library's pool, which holds them for the next call
+// until csrst_release_memory; larger ones go back to the driver.
+struct ScratchBuffer {
+  static constexpr size_t kKeep = (size_t)1 << 30;
+  void *p = nullptr;
+  explicit ScratchBuffer(cudaStream_t stream) : s(stream) {}
+  ScratchBuffer(const ScratchBuffer &) = delete;
+  ScratchBuffer &operator=(const ScratchBuffer &) = delete;
+  cudaError_t alloc(size_t bytes);
+  ~ScratchBuffer();
+
+ private:
+  cudaStream_t s;
+  bool pooled = false;
+};
+
 // api.cu: records the message csrst_get_error(NULL) returns and returns code
 // (for entry points that take no handle).
 int set_global_error(int code, const char *msg);
