@@ -20,8 +20,8 @@
 //     128, else of 2 or 4 tiles in turn, with 4 or 8 accumulators of BN
 //     columns in the 256 TMEM columns), hand it back through
 //     `acc_empty` after their read, add the biases and write FP32 and/or BF16
-//     outputs through affine index maps: as 16-byte runs through a 32 x 33
-//     staging block in shared memory where the map allows (below), else
+//     outputs through affine index maps: as 16-byte runs through a staging block
+//     in shared memory where the map allows (below), else
 //     element by element, a warp storing whole columns of its 32 rows (lanes
 //     on consecutive rows, straight from the registers) or, through the
 //     staging block, whole rows, whichever puts a warp's 32 stores next to
@@ -30,6 +30,16 @@
 // With two or more accumulators the epilogue of one tile overlaps the copies and
 // products of the next, and the copies run up to a ring ahead of the
 // products, so the kernel streams its operands and outputs at once.
+//
+// With K of a few hundred the launch is bound by the epilogue's own instructions
+// (tensor pipe 4 % busy, DRAM a sixth), which is what its form follows: two values
+// to an instruction where FP32 has a packed form, the tile's and maps' divisions as
+// a high product and a shift, the column bias as eight uniform 16-byte loads, row and
+// column runs staged 16 bytes at a time without bank conflicts.  100003 x 128 x 128
+// with bias, FP32 pre-activation and BF16 GELU output: 845 instructions a piece for
+// 1590 with one value at a time, shuffled biases and 64-bit divisions, 30.6 us for 39.4
+// (its 102 MB of inputs and outputs take 15.8 us at the measured copy rate); the values
+// are the same bit for bit.
 //
 // Waits on mbarriers are bounded (a launch parameter, csrst_gemm_set_wait_limit):
 // a wait that gives up sets *err = 1 and a shared flag that ends the other
@@ -157,6 +167,59 @@ __device__ __forceinline__ float gelu(float x) {
   return x < 0.0f ? h : x - h;
 }
 
+// Two FP32 values in one 64-bit register: the packed operations round each
+// half as the scalar ones do, at half the instructions.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t both(float a) { return pack2(a, a); }
+__device__ __forceinline__ float rcp_ftz(float a) {  // the values of __fdividef(1, a) for a >= 1
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
+// gelu() of two values, the same roundings: with h = |x| / 2 . 1 / p the result
+// is max(x, 0) - h on either side of zero.
+__device__ __forceinline__ void gelu2(float &x0, float &x1) {
+  const uint64_t w = pack2(fabsf(x0), fabsf(x1)), u = mul2(w, both(0.70710678118654752f));
+  uint64_t p = fma2(u, both(0.0000430638f), both(0.0002765672f));
+  p = fma2(u, p, both(0.0001520143f));
+  p = fma2(u, p, both(0.0092705272f));
+  p = fma2(u, p, both(0.0422820123f));
+  p = fma2(u, p, both(0.0705230784f));
+  p = fma2(u, p, both(1.0f));
+  p = mul2(p, p);
+  p = mul2(p, p);
+  p = mul2(p, p);
+  p = mul2(p, p);
+  float p0, p1;
+  unpack2(p, p0, p1);
+  const uint64_t h = mul2(mul2(w, both(0.5f)), pack2(rcp_ftz(p0), rcp_ftz(p1)));
+  unpack2(fma2(h, both(-1.0f), pack2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f))), x0, x1);
+}
+
 // Bounded wait of one thread that also gives up when another role has
 // failed (the shared flag, read every 64 polls).  Returns false on either;
 // a wait that ran out of polls raises the flag and sets *err = 1.
@@ -185,6 +248,17 @@ struct Seg {
   int amn;  // A is MN-major: element (m, k) of a batch at A[k * lda + m]
 };
 
+// Division of n < 2^31 by d >= 1 as a high product and a shift: m = floor(2^32
+// (2^l - d) / d) + 1 with l = ceil(log2 d) (Granlund and Montgomery 1994).
+struct Div {
+  uint32_t d, m, l;
+  __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(m, n) + n) >> l; }
+};
+Div make_div(int d) {
+  uint32_t l = 0;
+  while (l < 32 && (1ull << l) < (uint64_t)d) ++l;
+  return {(uint32_t)d, (uint32_t)((((1ull << l) - (uint64_t)d) << 32) / (uint64_t)d + 1), l};
+}
 
 // Everything one launch reads: the operand tensor maps (A1, B1, A2, B2;
 // 3-D over (K, rows, batch) where the operand has a batch stride, else
@@ -196,14 +270,28 @@ struct alignas(64) GemmArgs {
   csrst_gemm_epilogue ep;
   int *err;
   long long spin;
-  long long ntiles;
+  int ntiles;
+  Div dN, dM;                 // tile index -> column tile, row tile, batch
+  Div md, nd, tmd, tnd;       // the maps' divisors
   int nk1, nk2, M, N, tilesM, tilesN;
   int rank3[4];
   int amn[2];                 // per segment: A MN-major (two 64-row TMA boxes per stage)
   int o_mfast, t_mfast;
   int vec;
+  int bias4;                  // the column bias can be read as float4
   RunShape rs[4];             // pre, out32, out16 (primary map), out16t (second map)
   long long del[2][2][32];    // [map][rows, columns][i or j]
+};
+
+// Output tile t: first row and column, and the batch.
+struct Tile {
+  int m0, n0, z;
+  __device__ __forceinline__ Tile(const GemmArgs &a, int t, int bn) {
+    const uint32_t r = a.dN((uint32_t)t), zz = a.dM(r);
+    n0 = (t - (int)(r * a.dN.d)) * bn;
+    m0 = (int)(r - zz * a.dM.d) * kBM;
+    z = (int)zz;
+  }
 };
 
 // Row and column parts of an output map's index: z*sb + (m/md)*s0 + (m%md)*s1
@@ -213,6 +301,12 @@ __device__ __forceinline__ long long row_part(long long zb, int m, int md, long 
 }
 __device__ __forceinline__ long long col_part(int n, int nd, long long t0, long long t1) {
   return (long long)(n / nd) * t0 + (long long)(n % nd) * t1;
+}
+
+// The same with the divisions prepared.
+__device__ __forceinline__ long long map_part(int i, const Div &d, long long s0, long long s1) {
+  const uint32_t q = d((uint32_t)i);
+  return (long long)q * s0 + (long long)((uint32_t)i - q * d.d) * s1;
 }
 
 // One element under the primary map: residual, pre-activation, activation,
@@ -331,30 +425,122 @@ __device__ __forceinline__ void store_vec(const RunShape &rs, const float *st, c
   }
 }
 
+// Runs along the columns of a row (shape 0), the form of a row-major output:
+// each lane puts its row into the staging block as 16-byte pieces, the piece's
+// place XORed with the row so that neither side has a bank conflict, and the
+// warp stores whole rows' pieces: 24 memory instructions for 32 x 32 FP32 values
+// where one element at a time through the block takes 72.
+__device__ __forceinline__ void store_rows32(const float (&x)[32], float *st, const long long *rdel,
+                                             const long long *cdel, float *out, int lane) {
+  float4 *s4 = reinterpret_cast<float4 *>(st);
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    s4[lane * 8 + (c ^ (lane & 7))] = make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+  __syncwarp();
+  const int ch = lane & 7, r0 = lane >> 3;
+  out += cdel[4 * ch];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int row = 4 * k + r0;
+    *reinterpret_cast<float4 *>(out + rdel[row]) = s4[row * 8 + (ch ^ (row & 7))];
+  }
+}
+
+// The same for BF16 values, two to a word.
+__device__ __forceinline__ void store_rows16(const uint32_t (&w)[16], float *st, const long long *rdel,
+                                             const long long *cdel, __nv_bfloat16 *out, int lane) {
+  uint4 *s4 = reinterpret_cast<uint4 *>(st);
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    s4[lane * 4 + (c ^ ((lane >> 1) & 3))] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+  __syncwarp();
+  const int ch = lane & 3, r0 = lane >> 2;
+  out += cdel[8 * ch];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int row = 8 * k + r0;
+    *reinterpret_cast<uint4 *>(out + rdel[row]) = s4[row * 4 + (ch ^ ((row >> 1) & 3))];
+  }
+}
+
+// BF16 runs along the rows of a column (shape 1, a transposed output): the
+// block holds the piece by columns of 32 values.
+__device__ __forceinline__ void store_cols16(const uint32_t (&w)[16], float *st, const long long *rdel,
+                                             const long long *cdel, __nv_bfloat16 *out, int lane) {
+  uint16_t *s2 = reinterpret_cast<uint16_t *>(st);
+  const uint4 *s4 = reinterpret_cast<const uint4 *>(st);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    s2[(2 * j) * 32 + lane] = (uint16_t)(w[j] & 0xffffu);
+    s2[(2 * j + 1) * 32 + lane] = (uint16_t)(w[j] >> 16);
+  }
+  __syncwarp();
+  const int ch = lane & 3, c0 = lane >> 2;
+  out += rdel[8 * ch];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int col = 8 * k + c0;
+    *reinterpret_cast<uint4 *>(out + cdel[col]) = s4[col * 4 + ch];
+  }
+}
+
 // A whole 32 x 32 piece (lane = row, x[j] = column j, biases added) through
 // the vector forms: the pre-activation, then the activation, then the FP32
-// and BF16 copies, each from the warp's staging block.  obase / tbase: the
-// piece's base index under the primary and the second map.
+// and BF16 copies.  obase / tbase: the piece's base index under the primary and
+// the second map.
 __device__ __forceinline__ void store_piece_vec(const GemmArgs &a, const long long (*del)[2][32], float (&x)[32],
                                                 float *st, int lane, long long obase, long long tbase) {
   const csrst_gemm_epilogue &ep = a.ep;
-  if (ep.pre) {
+  auto stage = [&]() {  // the element-wise staging of the other shapes
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < 32; ++j) st[lane * 33 + j] = x[j];
     __syncwarp();
-    store_vec<4>(a.rs[0], st, del[0][0], del[0][1], ep.pre, obase, lane);
-    __syncwarp();
+  };
+  if (ep.pre) {
+    if (a.rs[0].shape == 0) {
+      store_rows32(x, st, del[0][0], del[0][1], ep.pre + obase, lane);
+    } else {
+      stage();
+      store_vec<4>(a.rs[0], st, del[0][0], del[0][1], ep.pre, obase, lane);
+    }
   }
   if (ep.act == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) x[j] = gelu(x[j]);
+    for (int j = 0; j < 32; j += 2) gelu2(x[j], x[j + 1]);
   }
+  if (ep.out32) {
+    if (a.rs[1].shape == 0) {
+      store_rows32(x, st, del[0][0], del[0][1], ep.out32 + obase, lane);
+    } else {
+      stage();
+      store_vec<4>(a.rs[1], st, del[0][0], del[0][1], ep.out32, obase, lane);
+    }
+  }
+  if (ep.out16 || ep.out16t) {
+    uint32_t w[16];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) st[lane * 33 + j] = x[j];
-  __syncwarp();
-  if (ep.out32) store_vec<4>(a.rs[1], st, del[0][0], del[0][1], ep.out32, obase, lane);
-  if (ep.out16) store_vec<8>(a.rs[2], st, del[0][0], del[0][1], ep.out16, obase, lane);
-  if (ep.out16t) store_vec<8>(a.rs[3], st, del[1][0], del[1][1], ep.out16t, tbase, lane);
+    for (int j = 0; j < 16; ++j) w[j] = bf16x2(x[2 * j], x[2 * j + 1]);
+#pragma unroll
+    for (int k = 2; k < 4; ++k) {
+      void *o = k == 2 ? ep.out16 : ep.out16t;
+      if (!o) continue;
+      const long long *rd = del[k - 2][0], *cd = del[k - 2][1];
+      const long long base = k == 2 ? obase : tbase;
+      __nv_bfloat16 *o16 = reinterpret_cast<__nv_bfloat16 *>(o);
+      if (a.rs[k].shape == 0) {
+        store_rows16(w, st, rd, cd, o16 + base, lane);
+      } else if (a.rs[k].shape == 1) {
+        store_cols16(w, st, rd, cd, o16 + base, lane);
+      } else {
+        stage();
+        store_vec<8>(a.rs[k], st, rd, cd, o, base, lane);
+      }
+    }
+  }
   __syncwarp();  // the staging block is free for the next piece
 }
 
@@ -406,9 +592,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
     if (lane == 0) {
       long long it = 0;  // stage fills issued
       bool ok = true;
-      for (long long t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
-        const long long r = t / a.tilesN;
-        const int n0 = (int)(t % a.tilesN) * BN, m0 = (int)(r % a.tilesM) * kBM, z = (int)(r / a.tilesM);
+      for (int t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
+        const Tile tile(a, t, BN);
+        const int n0 = tile.n0, m0 = tile.m0, z = tile.z;
         for (int kt = 0; kt < nk; ++kt) {
           const int s = (int)(it % G::STAGES);
           if (!wait_role(&empty[s], (uint32_t)((it / G::STAGES) & 1) ^ 1u, spin, fail, a.err)) {
@@ -445,7 +631,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
       long long it = 0;
       int lt = 0;
       bool ok = true, issued = false;
-      for (long long t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x, ++lt) {
+      for (int t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x, ++lt) {
         const int b = lt % G::NACC;
         if (!wait_role(&acc_empty[b], (uint32_t)((lt / G::NACC) & 1) ^ 1u, spin, fail, a.err)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -484,7 +670,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
     const csrst_gemm_epilogue &ep = a.ep;
     int lt = 0;
     bool first = true;
-    for (long long t = blockIdx.x; t < a.ntiles; t += gridDim.x, ++lt) {
+    for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, ++lt) {
       if (lt % G::TG != g) continue;
       const int b = lt % G::NACC;
       int ok = 1;
@@ -499,29 +685,53 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
       tmem_wait(v);
       asm volatile("tcgen05.fence::before_thread_sync;");
       mbar_arrive(&acc_empty[b]);  // this warp's read of the accumulator is done: hand it back
-      const long long r = t / a.tilesN;
-      const int n0 = (int)(t % a.tilesN) * BN, m0 = (int)(r % a.tilesM) * kBM, z = (int)(r / a.tilesM);
+      const Tile tile(a, t, BN);
+      const int n0 = tile.n0, m0 = tile.m0, z = tile.z;
       const int mrow = m0 + 32 * q, m = mrow + lane;
       const int ncol = n0 + c * 32, n = ncol + lane;
-      const long long orow = row_part((long long)z * ep.sb, m, ep.md, ep.sm0, ep.sm1);
-      const long long trow = ep.out16t ? row_part((long long)z * ep.tb, m, ep.tmd, ep.tm0, ep.tm1) : 0;
-      const long long ocol = col_part(n, ep.nd, ep.sn0, ep.sn1);
-      const long long tcol = ep.out16t ? col_part(n, ep.tnd, ep.tn0, ep.tn1) : 0;
       const float bm = (ep.bias_m && m < a.M) ? ep.bias_m[m] : 0.0f;
+      const uint64_t alpha = both(ep.alpha), bm2 = both(bm);
       float x[32];
-      if (ep.bias) {
-        const float bc = n < a.N ? ep.bias[n] : 0.0f;
+      const bool whole = a.vec && mrow + 32 <= a.M && ncol + 32 <= a.N;
+      if (ep.bias && whole && a.bias4) {
+        const float4 *b4 = reinterpret_cast<const float4 *>(ep.bias + ncol);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = ep.alpha * __uint_as_float(v[j]) + __shfl_sync(0xffffffffu, bc, j) + bm;
+        for (int j = 0; j < 8; ++j) {
+          const float4 bc = __ldg(b4 + j);
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int i = 4 * j + 2 * k;
+            unpack2(fma2(alpha, pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                         k ? pack2(bc.z, bc.w) : pack2(bc.x, bc.y)),
+                    x[i], x[i + 1]);
+          }
+        }
       } else {
+        const float bc = ep.bias && n < a.N ? ep.bias[n] : 0.0f;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = ep.alpha * __uint_as_float(v[j]) + bm;
+        for (int j = 0; j < 32; j += 2)
+          unpack2(fma2(alpha, pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])),
+                       ep.bias ? pack2(__shfl_sync(0xffffffffu, bc, j), __shfl_sync(0xffffffffu, bc, j + 1)) : bm2),
+                  x[j], x[j + 1]);
       }
-      if (a.vec && mrow + 32 <= a.M && ncol + 32 <= a.N)
-        store_piece_vec(a, s_del, x, st, lane, __shfl_sync(0xffffffffu, orow, 0) + __shfl_sync(0xffffffffu, ocol, 0),
-                        __shfl_sync(0xffffffffu, trow, 0) + __shfl_sync(0xffffffffu, tcol, 0));
-      else
+      if (ep.bias && ep.bias_m) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) unpack2(add2(pack2(x[j], x[j + 1]), bm2), x[j], x[j + 1]);
+      }
+      if (whole) {
+        store_piece_vec(
+            a, s_del, x, st, lane,
+            (long long)z * ep.sb + map_part(mrow, a.md, ep.sm0, ep.sm1) + map_part(ncol, a.nd, ep.sn0, ep.sn1),
+            ep.out16t ? (long long)z * ep.tb + map_part(mrow, a.tmd, ep.tm0, ep.tm1) +
+                            map_part(ncol, a.tnd, ep.tn0, ep.tn1)
+                      : 0);
+      } else {
+        const long long orow = row_part((long long)z * ep.sb, m, ep.md, ep.sm0, ep.sm1);
+        const long long trow = ep.out16t ? row_part((long long)z * ep.tb, m, ep.tmd, ep.tm0, ep.tm1) : 0;
+        const long long ocol = col_part(n, ep.nd, ep.sn0, ep.sn1);
+        const long long tcol = ep.out16t ? col_part(n, ep.tnd, ep.tn0, ep.tn1) : 0;
         store_piece(a, x, st, lane, mrow, ncol, orow, trow, ocol, tcol);
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -602,7 +812,16 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   a.N = N;
   a.tilesM = (M + kBM - 1) / kBM;
   a.tilesN = (N + BN - 1) / BN;
-  a.ntiles = (long long)batch * a.tilesM * a.tilesN;
+  if ((long long)batch * a.tilesM > 0x7fffffffll / a.tilesN) return CSRST_E_ARG;  // 2^31 tiles hold 2^43 outputs
+  a.ntiles = batch * a.tilesM * a.tilesN;
+  a.dN = make_div(a.tilesN);
+  a.dM = make_div(a.tilesM);
+  a.md = make_div(ep.md);
+  a.nd = make_div(ep.nd);
+  if (ep.out16t) {
+    a.tmd = make_div(ep.tmd);
+    a.tnd = make_div(ep.tnd);
+  }
   a.amn[0] = g0.amn;
   a.amn[1] = g1.amn;
   if (!encode_operand(&a.map[0], &a.rank3[0], g0.A, g0.nk * kBK, M, g0.lda, g0.sA, batch, kBM, g0.amn) ||
@@ -615,7 +834,8 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   a.o_mfast = rows_fast(ep.md, ep.nd, ep.sm0, ep.sm1, ep.sn0, ep.sn1, o_bytes);
   a.t_mfast = ep.out16t ? rows_fast(ep.tmd, ep.tnd, ep.tm0, ep.tm1, ep.tn0, ep.tn1, 2) : 0;
   vector_forms(a, M, N, batch);
-  const long long grid = a.ntiles < sms ? a.ntiles : sms;
+  a.bias4 = ep.bias && !(reinterpret_cast<uintptr_t>(ep.bias) & 15);
+  const int grid = a.ntiles < sms ? a.ntiles : sms;
   k_gemm<BN><<<(unsigned)grid, kThreads, G::SMEM, s>>>(a);
   return cudaGetLastError() == cudaSuccess ? CSRST_OK : CSRST_E_CUDA;
 }
