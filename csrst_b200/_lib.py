@@ -88,6 +88,9 @@ def lib():
         "csrst_nn_adam": ([P, P, P, P, C.c_longlong, P, C.c_float, C.c_float, C.c_float, P], C.c_int),
         "csrst_nn_spectral_pack": ([P, P, C.c_int, C.c_int, P, P, P], C.c_int),
         "csrst_nn_spectral_unpack": ([P, C.c_int, C.c_int, P, P, P], C.c_int),
+        "csrst_fno_forward": ([P, P, P, P, P], C.c_int),
+        "csrst_fno_backward": ([P, P, P, P, P, P], C.c_int),
+        "csrst_fno_refresh": ([P, C.c_longlong, P], C.c_int),
         "csrst_get_particles": ([P, D, D, D, D], C.c_int),
         "csrst_get_old_positions": ([P, D, D], C.c_int),
         "csrst_get_window": ([P, I, D, I], C.c_int),

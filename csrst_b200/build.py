@@ -1,4 +1,4 @@
-"""Builds libcsrst_gpu.so in this directory from csrc/*.cu for sm_100a.
+"""Builds libcsrst_gpu.so in this directory from csrc for sm_100a.
 
 The FP64 kernels are compiled with --fmad=false: every multiply and add is
 rounded separately, as in the reference's x86-64 build, which is what makes
@@ -13,7 +13,7 @@ from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 SRC = ["api.cu", "geometry.cu", "particles.cu", "particles32.cu", "fields.cu", "diag.cu", "poisson.cu",
-       "gemm.cu", "nn.cu", "noalloc.cu"]
+       "gemm.cu", "nn.cu", "fno.cpp", "noalloc.cu"]
 FMA_ON = {"particles32.cu", "gemm.cu", "nn.cu"}
 OUT = HERE / "libcsrst_gpu.so"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

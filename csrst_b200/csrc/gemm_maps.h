@@ -71,7 +71,8 @@ inline bool piece_offsets(const MapDesc &d, long long *rdel, long long *cdel) {
   return true;
 }
 
-inline long long mod_pos(long long a, long long m) { return ((a % m) + m) % m; }
+// a mod m for a power of two m (the run lengths and the sectors' sizes).
+inline long long mod_pos(long long a, long long m) { return a & (m - 1); }
 
 // Every piece's base index a multiple of L (16 bytes) and the output 16-byte
 // aligned.  A piece starts at row 32p: its row part advances by (32 / md) s0
@@ -114,7 +115,7 @@ inline RunShape run_shape(const long long *rdel, const long long *cdel, int L) {
         for (int r = 0; r < 32; ++r) {
           const int oi = (f ? r / nj : r % ni) * ri, oj = (f ? r % nj : r / ni) * rj;
           const long long b = (rdel[oi] + cdel[oj]) * (16 / L);
-          const long long s = (b - mod_pos(b, unit)) / unit;
+          const long long s = (b - mod_pos(b, unit)) >> (unit == 32 ? 5 : 7);
           bool seen = false;
           for (int q = 0; q < k; ++q) seen |= seen_at[q] == s;
           if (!seen) seen_at[k++] = s;

@@ -33,7 +33,7 @@ import numpy as np
 import torch
 
 from ._lib import CsrstError, lib
-from .tensor import check_errors, gemm, gemm_dual, rowmap
+from .tensor import _err, check_errors
 
 NBINS, NFEAT = 256, 64
 KSPLIT = 256          # K-columns per partial product of a weight gradient
@@ -75,6 +75,20 @@ def _stream():
 def _ck(rc, what):
     if rc:
         raise CsrstError(rc, what)
+
+
+class _Net(C.Structure):
+    """csrst_fno (include/csrst.h): one network's device pointers and one batch size's buffers."""
+    _fields_ = ([(k, C.c_int) for k in ("width", "modes", "layers", "nout", "batch", "train")] +
+                [(k, C.c_void_p) for k in (
+                    "w", "g", "w16", "WT16", "Mk16", "MkT16", "Q1T16", "Q2T16", "F16", "FT16", "G16", "GT16", "V16",
+                    "U16", "Z16", "Zp16", "A1_16", "out", "Vg16", "Ut16", "Hfull", "A1pre", "A1t16", "Xt16", "dOut",
+                    "dOut16", "dOutT16", "dA1", "dH", "dH16", "dHt16", "dV", "dVn", "dZ16", "dZt16", "dSk16", "dS16",
+                    "dMk", "part", "cpart", "lpart", "loss")])
+
+
+def _ptrs(ts):
+    return (C.c_void_p * max(len(ts), 1))(*[t.data_ptr() for t in ts])
 
 
 class _Buffers:
@@ -198,16 +212,24 @@ class FNO:
     def refresh(self):
         """BF16 copies of the weights: one cast of the flat buffer, then the
         transposed pointwise weights and the block-packed spectral weights."""
-        L, w, s = self.layers, self.width, _stream()
-        _ck(lib().csrst_nn_cast_bf16(_p(self.w), _p(self.w16), self.n, s), "cast")
-        for l in range(L):
-            _ck(lib().csrst_nn_transpose_bf16(_p(self.view("W%d" % l, self.w16)), _p(self.WT16[l]), 1, w, w, w, s),
-                "transpose")
-            _ck(lib().csrst_nn_spectral_pack(_p(self.view("Wr%d" % l)), _p(self.view("Wi%d" % l)), self.modes, w,
-                                             _p(self.Mk16[l]), _p(self.MkT16[l]), s), "spectral pack")
-        _ck(lib().csrst_nn_transpose_bf16(_p(self.view("Q1", self.w16)), _p(self.Q1T16), 1, w, w, w, s), "transpose")
-        _ck(lib().csrst_nn_transpose_bf16(_p(self.view("Q2", self.w16)), _p(self.Q2T16), 1, self.nout, w, 64, s),
-            "transpose")
+        _ck(lib().csrst_fno_refresh(C.byref(self._net()), self.n, _stream()), "refresh")
+
+    def _net(self, bf=None, B=1):
+        """The C structure of this network and of the buffers of a batch of B members, for one call."""
+        n = _Net(self.width, self.modes, self.layers, self.nout, B, 1 if bf is not None and bf.train else 0)
+        for k in ("w", "g", "w16", "Q1T16", "Q2T16", "F16", "FT16", "G16", "GT16"):
+            setattr(n, k, getattr(self, k).data_ptr())
+        n.keep = [_ptrs(v) for v in (self.WT16, self.Mk16, self.MkT16)]
+        n.WT16, n.Mk16, n.MkT16 = map(C.addressof, n.keep)
+        if bf is not None:
+            for k, v in vars(bf).items():
+                if isinstance(v, list):
+                    v = _ptrs(v)
+                    n.keep.append(v)
+                    setattr(n, k, C.addressof(v))
+                elif k != "train":
+                    setattr(n, k, v.data_ptr())
+        return n
 
     def _buf(self, B, train):
         key = (B, train)
@@ -216,47 +238,9 @@ class FNO:
         return self._bufs[key]
 
     # ---- forward ----
-    def _tr16(self, src, dst, batch, rows, cols, ldd=None):
-        _ck(lib().csrst_nn_transpose_bf16(_p(src), _p(dst), batch, rows, cols, ldd or rows, _stream()), "transpose")
-
-    def _tr32(self, src, dst, rows, cols):
-        _ck(lib().csrst_nn_transpose_b32(_p(src), _p(dst), 1, rows, cols, rows, _stream()), "transpose")
-
-    def _forward(self, bf, B, X16, out=None):
-        w, m, L, R = self.width, self.modes, self.layers, B * NBINS
-        tr = bf.train
-        w16 = lambda n: self.view(n, self.w16)
-        # lift: V0 in rows and in per-member channel rows
-        gemm(X16, w16("P"), R, w, NFEAT, bias=self.view("p"), out16=bf.V16[0])
-        for l in range(L):
-            i, o = (l, l + 1) if tr else (l & 1, (l + 1) & 1)
-            if tr:
-                self._tr16(bf.V16[i], bf.Vg16[i], 1, R, w)
-            # forward DFT over the bins, per member b: rows c of V[b] read MN-major (the
-            # bins are V's rows) -> U[k][b][2c + ri]
-            gemm(bf.V16[i], self.F16, w, 2 * m, NBINS, a_mn=True, lda=w, batch=B, stride_a=NBINS * w,
-                 out16=bf.U16, omap=dict(md=1, nd=2, sm0=2, sm1=0, sn0=2 * w * B, sn1=1), sb=2 * w)
-            if tr:
-                self._tr16(bf.U16, bf.Ut16[l], m, B, 2 * w)
-            # mode mixing: per mode k, Z[b][2o + p] = sum U[b][2c + q] Mk[2o + p][2c + q]
-            gemm(bf.U16, self.Mk16[l], B, 2 * w, 2 * w, batch=m, stride_a=2 * w * B, stride_b=4 * w * w,
-                 out16=bf.Z16, omap=rowmap(2 * w), sb=2 * w * B)
-            # (mode, (member, channel)) pairs -> ((member, channel), mode) pairs: Zp[(b, o)][2k + p]
-            self._tr32(bf.Z16, bf.Zp16, m, B * w)
-            # per member b, one accumulator: H_b[o][n] = sum_j Zp[(b, o)][j] G[n][j]   (truncated inverse DFT)
-            #                                          + sum_c W[o][c] V[b][n][c]    (pointwise product)
-            # + bias[o]; pre-activation, activation, V in rows and in per-member channel rows
-            act = l < L - 1
-            gemm_dual(bf.Zp16, self.G16, 2 * m, w16("W%d" % l), bf.V16[i], w, w, NBINS, stride_a1=2 * m * w,
-                      stride_b2=NBINS * w, batch=B, bias_m=self.view("b%d" % l),
-                      pre=bf.Hfull[l] if (tr and act) else None, act=1 if act else 0, out16=bf.V16[o],
-                      omap=dict(md=1, nd=1, sm0=1, sm1=0, sn0=w, sn1=0), sb=NBINS * w)
-        Vl = bf.V16[L if tr else L & 1]
-        if tr:
-            self._tr16(Vl, bf.Vg16[L], 1, R, w)
-        gemm(Vl, w16("Q1"), R, w, w, bias=self.view("q1"), act=1, pre=bf.A1pre if tr else None, out16=bf.A1_16,
-             out16t=bf.A1t16 if tr else None, tmap=dict(md=1, nd=1, sm0=1, sm1=0, sn0=R, sn1=0))
-        gemm(bf.A1_16, w16("Q2"), R, self.nout, w, bias=self.view("q2"), out32=bf.out if out is None else out)
+    def _forward(self, net, X16, out):
+        assert X16.dtype == torch.bfloat16
+        _ck(lib().csrst_fno_forward(C.byref(net), _p(X16), _p(out), _p(_err(self.device)), _stream()), "forward")
 
     def predict(self, X, chunk=4096):
         """X: [N][256][64] BF16 (device) -> wake [N][256][nout] FP32 (device), in chunks of members."""
@@ -265,76 +249,10 @@ class FNO:
         for a in range(0, N, chunk):
             B = min(chunk, N - a)
             bf = self._buf(B, False)
-            self._forward(bf, B, X[a:a + B].reshape(B * NBINS, NFEAT), out[a:a + B])
+            self._forward(self._net(bf, B), X[a:a + B].reshape(B * NBINS, NFEAT), out[a:a + B])
         return out
 
     # ---- backward ----
-    def _wgrad(self, bf, At, Bt, M, N, K, name):
-        """grad[name][M][N] = At[M][K] Bt[N][K]^T as KSPLIT-column partial
-        products summed in order."""
-        S = K // KSPLIT
-        gemm(At, Bt, M, N, KSPLIT, lda=K, ldb=K, batch=S, stride_a=KSPLIT, stride_b=KSPLIT, out32=bf.part,
-             omap=rowmap(N), sb=M * N)
-        self._colsum(bf, bf.part, S, M * N, self.view(name, self.g))
-
-    def _colsum(self, bf, x, rows, cols, out, accumulate=False):
-        assert bf.cpart.numel() >= ((rows + 255) // 256) * cols
-        _ck(lib().csrst_nn_colsum(_p(x), rows, cols, _p(bf.cpart), _p(out), 1 if accumulate else 0, _stream()),
-            "colsum")
-
-    def _backward(self, bf, B, X16, T, Wt=None):
-        w, m, L, R, nout = self.width, self.modes, self.layers, B * NBINS, self.nout
-        s = _stream()
-        lb = lib()
-        w16 = lambda n: self.view(n, self.w16)
-        # loss and dLoss/dout into the first nout columns of a 64-column buffer
-        _ck(lb.csrst_nn_mse(_p(bf.out), _p(T), _p(Wt), R * nout, _p(bf.dOut), nout, 64, 1, _p(bf.lpart),
-                            _p(bf.loss), s), "mse")
-        _ck(lb.csrst_nn_cast_bf16(_p(bf.dOut), _p(bf.dOut16), R * 64, s), "cast")
-        _ck(lb.csrst_nn_transpose_bf16(_p(bf.dOut16), _p(bf.dOutT16), 1, R, 64, R, s), "transpose")
-        self._wgrad(bf, bf.dOutT16, bf.A1t16, nout, w, R, "Q2")
-        self._colsum(bf, bf.dOut, R, 64, self.view("q2", self.g))  # q2 and the padding after it
-        gemm(bf.dOut16, self.Q2T16, R, w, 64, out32=bf.dA1)
-        _ck(lb.csrst_nn_gelu_bwd(_p(bf.dA1), _p(bf.A1pre), _p(bf.dH), _p(bf.dH16), R * w, s), "gelu")
-        _ck(lb.csrst_nn_transpose_bf16(_p(bf.dH16), _p(bf.dHt16), 1, R, w, R, s), "transpose")
-        self._wgrad(bf, bf.dHt16, bf.Vg16[L], w, w, R, "Q1")
-        self._colsum(bf, bf.dH, R, w, self.view("q1", self.g))
-        gemm(bf.dH16, self.Q1T16, R, w, w, out32=bf.dV)
-        dV, dVn = bf.dV, bf.dVn
-        for l in reversed(range(L)):
-            if l < L - 1:
-                _ck(lb.csrst_nn_gelu_bwd(_p(dV), _p(bf.Hfull[l]), _p(bf.dH), _p(bf.dH16), R * w, s), "gelu")
-                dH = bf.dH
-            else:
-                _ck(lb.csrst_nn_cast_bf16(_p(dV), _p(bf.dH16), R * w, s), "cast")
-                dH = dV
-            _ck(lb.csrst_nn_transpose_bf16(_p(bf.dH16), _p(bf.dHt16), 1, R, w, R, s), "transpose")
-            self._wgrad(bf, bf.dHt16, bf.Vg16[l], w, w, R, "W%d" % l)
-            self._colsum(bf, dH, R, w, self.view("b%d" % l, self.g))
-            # adjoint of the inverse DFT: dZ[k][(o, ri)][b] = sum_n dH[b][n][o] G[n][2k + ri] (rows (o, b) of dH^T)
-            gemm(bf.dHt16, self.GT16, w * B, 2 * m, NBINS, out16=bf.dZt16,
-                 omap=dict(md=B, nd=2, sm0=2 * B, sm1=1, sn0=2 * w * B, sn1=B))
-            self._tr16(bf.dZt16, bf.dZ16, m, 2 * w, B)
-            # mode-mixing weights: dMk[k] = dZ_k^T U_k, then back to (dWr, dWi)
-            gemm(bf.dZt16, bf.Ut16[l], 2 * w, 2 * w, B, batch=m, stride_a=2 * w * B, stride_b=2 * w * B,
-                 out32=bf.dMk, omap=rowmap(2 * w), sb=4 * w * w)
-            _ck(lb.csrst_nn_spectral_unpack(_p(bf.dMk), m, w, _p(self.view("Wr%d" % l, self.g)),
-                                            _p(self.view("Wi%d" % l, self.g)), s), "spectral unpack")
-            # dU_k = dZ_k Mk -> dSk[k][b][2c + q] -> dS[(b, c)][2k + q]
-            gemm(bf.dZ16, self.MkT16[l], B, 2 * w, 2 * w, batch=m, stride_a=2 * w * B, stride_b=4 * w * w,
-                 out16=bf.dSk16, omap=rowmap(2 * w), sb=2 * w * B)
-            self._tr32(bf.dSk16, bf.dS16, m, B * w)
-            # input gradient: pointwise part, then the adjoint of the forward DFT added on
-            gemm(bf.dH16, self.WT16[l], R, w, w, out32=dVn)
-            gemm(bf.dS16, self.FT16, B * w, NBINS, 2 * m, out32=dVn, accumulate=True,
-                 omap=dict(md=w, nd=1, sm0=NBINS * w, sm1=1, sn0=w, sn1=0))
-            dV, dVn = dVn, dV
-        _ck(lb.csrst_nn_cast_bf16(_p(dV), _p(bf.dH16), R * w, s), "cast")
-        _ck(lb.csrst_nn_transpose_bf16(_p(bf.dH16), _p(bf.dHt16), 1, R, w, R, s), "transpose")
-        _ck(lb.csrst_nn_transpose_bf16(_p(X16), _p(bf.Xt16), 1, R, NFEAT, R, s), "transpose")
-        self._wgrad(bf, bf.dHt16, bf.Xt16, w, NFEAT, R, "P")
-        self._colsum(bf, dV, R, w, self.view("p", self.g))
-
     def loss_and_grad(self, X, T, weight=None):
         """X: [B][256][64] BF16, T: [B][256][nout] FP32 (device, B a multiple
         of 64), weight: optional FP32 per-output weights of the squared error
@@ -345,9 +263,12 @@ class FNO:
             raise ValueError("training batches must be a multiple of 64 members")
         bf = self._buf(B, True)
         X16 = X.reshape(B * NBINS, NFEAT)
-        self._forward(bf, B, X16)
-        self._backward(bf, B, X16, T.reshape(B * NBINS, self.nout),
-                       None if weight is None else weight.reshape(B * NBINS, self.nout))
+        T = T.reshape(B * NBINS, self.nout)
+        Wt = None if weight is None else weight.reshape(B * NBINS, self.nout)
+        net = self._net(bf, B)
+        self._forward(net, X16, bf.out)
+        _ck(lib().csrst_fno_backward(C.byref(net), _p(X16), _p(T), _p(Wt), _p(_err(self.device)), _stream()),
+            "backward")
         return bf.loss
 
     def adam(self, lr0=1e-3, lr_min=1e-5, total=10000, b1=0.9, b2=0.999, eps=1e-8):

@@ -301,6 +301,44 @@ int csrst_nn_adam(float *w, const float *g, float *m, float *v, long long n, con
 int csrst_nn_spectral_pack(const float *wr, const float *wi, int modes, int ch, void *mk, void *mkt, void *stream);
 int csrst_nn_spectral_unpack(const float *dmk, int modes, int ch, float *dwr, float *dwi, void *stream);
 
+/* The wake surrogate (a 1D Fourier neural operator over 256 bins of 64 features) as launch sequences
+ * of the products and kernels above: the device pointers of one network and of the buffers of one
+ * batch size, read during the call only.  w, g, w16: the flat parameters (FP32), their gradient and
+ * BF16 copy in the order P [width][64], p, per layer W [width][width], b, Wr and Wi
+ * [modes][width][width], then Q1, q1, Q2 [nout][width], q2.  Fields from Vg16 on are read with train != 0 alone.
+ * R = 256 batch rows. */
+typedef struct {
+  int width, modes, layers, nout, batch, train;
+  const float *w;
+  float *g;
+  void *w16;
+  void *const *WT16, *const *Mk16, *const *MkT16;    /* per layer: W^T, block matrices and their transposes */
+  void *Q1T16, *Q2T16;                               /* Q1^T, Q2^T [width][64] */
+  const void *F16, *FT16, *G16, *GT16;               /* DFT matrices [2 modes][256], [256][2 modes] */
+  void *const *V16;                                  /* layers + 1 when training, else 2: [R][width] */
+  void *U16, *Z16, *Zp16, *A1_16;                    /* spectra [modes][batch][2 width] ..., [R][width] */
+  float *out;                                        /* [R][nout], the training pass's output */
+  void *const *Vg16, *const *Ut16;                   /* layers + 1: [width][R]; layers: [modes][2 width][batch] */
+  float *const *Hfull;                               /* layers - 1: [R][width] pre-activations */
+  float *A1pre;
+  void *A1t16, *Xt16;
+  float *dOut;                                       /* [R][64], columns from nout on zero */
+  void *dOut16, *dOutT16;
+  float *dA1, *dH;
+  void *dH16, *dHt16;
+  float *dV, *dVn;
+  void *dZ16, *dZt16, *dSk16, *dS16;
+  float *dMk;                                        /* [modes][2 width][2 width] */
+  float *part, *cpart;                               /* partial products, column-sum scratch */
+  double *lpart, *loss;                              /* 256 doubles of scratch, the loss */
+} csrst_fno;
+/* out [R][nout] (FP32) for X16 [R][64] (BF16); *err as for the GEMM */
+int csrst_fno_forward(const csrst_fno *f, const void *X16, float *out, int *err, void *stream);
+/* after a training forward pass into f->out: loss and the whole gradient g (T, Wt: [R][nout]; Wt may be NULL) */
+int csrst_fno_backward(const csrst_fno *f, const void *X16, const float *T, const float *Wt, int *err, void *stream);
+/* w16 and the transposed and block-packed copies of the n parameters w (batch: any positive number) */
+int csrst_fno_refresh(const csrst_fno *f, long long n, void *stream);
+
 /* Beam moments (PartBunch::calcBeamParameters, PartBunch.cpp:584-657):
  * out18 = rmean2, pmean2, rrms2, prms2, eps_norm2, rmin2, rmax2, Ekin[MeV], dE, Dy, DDy. */
 int csrst_diag_moments(csrst_handle *h, double *out18);
