@@ -2,16 +2,17 @@
 // backward pass and the refresh of its BF16 weight copies as one host call
 // each, over the GEMM (gemm.cu) and the element-wise kernels (nn.cu).
 //
-// A forward pass is 22 launches and a training step 106, of 5 to 30 us each at
+// A forward pass is 22 launches and a training step about 90, of 3 to 30 us each at
 // small batches, so a host that takes longer than that per launch is what
 // bounds them: from Python, at 23 us a launch (argument structures, views,
 // foreign calls), the wake of 37 bunches took 494 us and a 64-member training
 // step 1754 us, where the same launches replayed as a graph took 141 and 972 us.  From
-// here a launch costs its tensor maps and the launch itself: 163 and 1155 us.
-// Nothing is kept between calls: every pointer comes in with the call.
+// here a launch costs its tensor maps and the launch itself: 163 and 1155 us with
+// the kernels as they were then.  Nothing is kept between calls: every pointer comes in with the call.
 #include <stdint.h>
 
 #include "../../include/csrst.h"
+#include "nn.h"
 
 namespace {
 
@@ -91,8 +92,9 @@ struct Seq {
   void colsum(const float *x, long long rows, long long cols, float *out) {
     if (ok()) ck(csrst_nn_colsum(x, (int)rows, (int)cols, f.cpart, out, 0, s));
   }
-  void gelu_bwd(const float *dy, const float *pre) {
-    if (ok()) ck(csrst_nn_gelu_bwd(dy, pre, f.dH, f.dH16, R * w, s));
+  // dy through the activation (pre NULL: none) as dx32, dH16 and dHt16
+  void activation_bwd(const float *dy, const float *pre, float *dx32) {
+    if (ok()) ck(csrst::nn_backward_rows(dy, pre, dx32, f.dH16, f.dHt16, (int)R, (int)w, s));
   }
   // grad[M][N] = At[M][R] Bt[N][R]^T as kSplit-column partial products summed in order
   void wgrad(const void *At, const void *Bt, long long M, long long N, float *out) {
@@ -170,29 +172,22 @@ void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
   // loss and dLoss/dout into the first nout columns of a 64-column buffer
   if (q.ok())
     q.ck(csrst_nn_mse(f.out, T, Wt, R * nout, f.dOut, (int)nout, 64, 1, f.lpart, f.loss, q.s));
-  q.cast(f.dOut, f.dOut16, R * 64);
-  q.transpose16(f.dOut16, f.dOutT16, 1, R, 64, R);
+  if (q.ok()) q.ck(csrst::nn_backward_rows(f.dOut, nullptr, nullptr, f.dOut16, f.dOutT16, (int)R, 64, q.s));
   q.wgrad(f.dOutT16, f.A1t16, nout, w, q.g32(q.oQ2()));
   q.colsum(f.dOut, R, 64, q.g32(q.oq2()));  // q2 and the padding after it
   ep = epilogue(rows_of(w));
   ep.out32 = f.dA1;
   q.gemm(f.dOut16, f.Q2T16, R, w, 64, ep);
-  q.gelu_bwd(f.dA1, f.A1pre);
-  q.transpose16(f.dH16, f.dHt16, 1, R, w, R);
+  q.activation_bwd(f.dA1, f.A1pre, f.dH);
   q.wgrad(f.dHt16, f.Vg16[f.layers], w, w, q.g32(q.oQ1()));
   q.colsum(f.dH, R, w, q.g32(q.oq1()));
   ep.out32 = f.dV;
   q.gemm(f.dH16, f.Q1T16, R, w, w, ep);
   float *dV = f.dV, *dVn = f.dVn;
   for (int l = f.layers - 1; l >= 0; --l) {
-    const float *dH = dV;
-    if (l < f.layers - 1) {
-      q.gelu_bwd(dV, f.Hfull[l]);
-      dH = f.dH;
-    } else {
-      q.cast(dV, f.dH16, R * w);
-    }
-    q.transpose16(f.dH16, f.dHt16, 1, R, w, R);
+    const bool act = l < f.layers - 1;
+    const float *dH = act ? f.dH : dV;
+    q.activation_bwd(dV, act ? f.Hfull[l] : nullptr, act ? f.dH : nullptr);
     q.wgrad(f.dHt16, f.Vg16[l], w, w, q.g32(q.oW(l)));
     q.colsum(dH, R, w, q.g32(q.ob(l)));
     // adjoint of the inverse DFT: dZ[k][(o, ri)][b] = sum_n dH[b][n][o] G[n][2k + ri] (rows (o, b) of dH^T)
@@ -223,8 +218,7 @@ void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
     dV = dVn;
     dVn = t;
   }
-  q.cast(dV, f.dH16, R * w);
-  q.transpose16(f.dH16, f.dHt16, 1, R, w, R);
+  q.activation_bwd(dV, nullptr, nullptr);
   q.transpose16(X16, f.Xt16, 1, R, kFeat, R);
   q.wgrad(f.dHt16, f.Xt16, w, kFeat, q.g32(q.oP()));
   q.colsum(dV, R, w, q.g32(q.op()));

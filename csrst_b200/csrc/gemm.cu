@@ -52,6 +52,7 @@
 #include <stdint.h>
 
 #include "../../include/csrst.h"
+#include "chain.cuh"
 #include "gemm_maps.h"
 #include "tma.cuh"
 
@@ -561,6 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
   const bool stuck = a.spin < 0;
   const long long spin = stuck ? -a.spin : a.spin;
 
+  chain_next();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                  "r"(G::TMEM_COLS));
@@ -584,6 +586,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
+  chain_wait();
   const uint32_t tmem = tmem_base;
   const int nk = a.nk1 + a.nk2;
 
@@ -697,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
         const float4 *b4 = reinterpret_cast<const float4 *>(ep.bias + ncol);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float4 bc = __ldg(b4 + j);
+          const float4 bc = b4[j];
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             const int i = 4 * j + 2 * k;
@@ -836,8 +839,7 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   vector_forms(a, M, N, batch);
   a.bias4 = ep.bias && !(reinterpret_cast<uintptr_t>(ep.bias) & 15);
   const int grid = a.ntiles < sms ? a.ntiles : sms;
-  k_gemm<BN><<<(unsigned)grid, kThreads, G::SMEM, s>>>(a);
-  return cudaGetLastError() == cudaSuccess ? CSRST_OK : CSRST_E_CUDA;
+  return launch_chained(k_gemm<BN>, dim3(grid), dim3(kThreads), G::SMEM, s, a) ? CSRST_OK : CSRST_E_CUDA;
 }
 
 bool seg_ok(const void *A, long long lda, long long sa, const void *B, long long ldb, long long sb, int K) {
