@@ -37,7 +37,7 @@
 // a high product and a shift, the column bias as eight uniform 16-byte loads, row and
 // column runs staged 16 bytes at a time without bank conflicts.  100003 x 128 x 128
 // with bias, FP32 pre-activation and BF16 GELU output: 845 instructions a piece for
-// 1590 with one value at a time, shuffled biases and 64-bit divisions, 30.6 us for 39.4
+// 1590 with one value at a time, shuffled biases and 64-bit divisions, 27.3 us for 39.3
 // (its 102 MB of inputs and outputs take 15.8 us at the measured copy rate); the values
 // are the same bit for bit.
 //
@@ -50,6 +50,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "../../include/csrst.h"
 #include "chain.cuh"
@@ -265,7 +267,7 @@ Div make_div(int d) {
 // 3-D over (K, rows, batch) where the operand has a batch stride, else
 // 2-D), the epilogue, the tile grid, the sweep orders of the two maps and
 // their vector forms (vec: every output of the launch has one and there is
-// no residual or accumulation).
+// no residual).
 struct alignas(64) GemmArgs {
   CUtensorMap map[4];
   csrst_gemm_epilogue ep;
@@ -328,9 +330,14 @@ __device__ __forceinline__ float finish(const csrst_gemm_epilogue &ep, long long
 // goes through the warp's staging block st[32][33] (conflict-free both ways)
 // and the warp stores a row per instruction.
 __device__ __forceinline__ void store_piece(const GemmArgs &a, float (&x)[32], float *st, int lane, int mrow, int ncol,
-                                            long long orow, long long trow, long long ocol, long long tcol) {
+                                            int z) {
   const csrst_gemm_epilogue &ep = a.ep;
-  const bool mok = mrow + lane < a.M, nok = ncol + lane < a.N;
+  const int m = mrow + lane, n = ncol + lane;
+  const long long orow = row_part((long long)z * ep.sb, m, ep.md, ep.sm0, ep.sm1);
+  const long long trow = ep.out16t ? row_part((long long)z * ep.tb, m, ep.tmd, ep.tm0, ep.tm1) : 0;
+  const long long ocol = col_part(n, ep.nd, ep.sn0, ep.sn1);
+  const long long tcol = ep.out16t ? col_part(n, ep.tnd, ep.tn0, ep.tn1) : 0;
+  const bool mok = m < a.M, nok = n < a.N;
   if (a.o_mfast) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -374,6 +381,13 @@ __device__ __forceinline__ void store_piece(const GemmArgs &a, float (&x)[32], f
     }
   }
   __syncwarp();  // the staging block is free for the next piece
+}
+
+// The same out of line, for the ragged edge pieces of launches whose other pieces
+// all have a vector form: their registers and code stay out of that kernel's way.
+__device__ __noinline__ void store_piece_cold(const GemmArgs &a, float (&x)[32], float *st, int lane, int mrow,
+                                              int ncol, int z) {
+  store_piece(a, x, st, lane, mrow, ncol, z);
 }
 
 // Row and column offsets of element t of a run of shape S, and the run's
@@ -426,11 +440,28 @@ __device__ __forceinline__ void store_vec(const RunShape &rs, const float *st, c
   }
 }
 
+// *at(k) += of(k) for a lane's eight runs, the reads four at a time.
+template <class At, class Of>
+__device__ __forceinline__ void add_runs(At at, Of of) {
+#pragma unroll
+  for (int h = 0; h < 8; h += 4) {
+    float4 o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = *reinterpret_cast<const float4 *>(at(h + k));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 v = of(h + k);
+      *reinterpret_cast<float4 *>(at(h + k)) = make_float4(o[k].x + v.x, o[k].y + v.y, o[k].z + v.z, o[k].w + v.w);
+    }
+  }
+}
+
 // Runs along the columns of a row (shape 0), the form of a row-major output:
 // each lane puts its row into the staging block as 16-byte pieces, the piece's
 // place XORed with the row so that neither side has a bank conflict, and the
 // warp stores whole rows' pieces: 24 memory instructions for 32 x 32 FP32 values
 // where one element at a time through the block takes 72.
+template <bool ADD>
 __device__ __forceinline__ void store_rows32(const float (&x)[32], float *st, const long long *rdel,
                                              const long long *cdel, float *out, int lane) {
   float4 *s4 = reinterpret_cast<float4 *>(st);
@@ -441,6 +472,11 @@ __device__ __forceinline__ void store_rows32(const float (&x)[32], float *st, co
   __syncwarp();
   const int ch = lane & 7, r0 = lane >> 3;
   out += cdel[4 * ch];
+  if constexpr (ADD) {
+    add_runs([&](int k) { return out + rdel[4 * k + r0]; },
+             [&](int k) { return s4[(4 * k + r0) * 8 + (ch ^ ((4 * k + r0) & 7))]; });
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int row = 4 * k + r0;
@@ -466,8 +502,29 @@ __device__ __forceinline__ void store_rows16(const uint32_t (&w)[16], float *st,
   }
 }
 
-// BF16 runs along the rows of a column (shape 1, a transposed output): the
-// block holds the piece by columns of 32 values.
+// Runs along the rows of a column (shape 1, a transposed output): the block
+// holds the piece by columns of 32 values.
+template <bool ADD>
+__device__ __forceinline__ void store_cols32(const float (&x)[32], float *st, const long long *rdel,
+                                             const long long *cdel, float *out, int lane) {
+  const float4 *s4 = reinterpret_cast<const float4 *>(st);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 32; ++j) st[j * 32 + lane] = x[j];
+  __syncwarp();
+  const int ch = lane & 7, c0 = lane >> 3;
+  out += rdel[4 * ch];
+  if constexpr (ADD) {
+    add_runs([&](int k) { return out + cdel[4 * k + c0]; }, [&](int k) { return s4[(4 * k + c0) * 8 + ch]; });
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int col = 4 * k + c0;
+    *reinterpret_cast<float4 *>(out + cdel[col]) = s4[col * 8 + ch];
+  }
+}
+
 __device__ __forceinline__ void store_cols16(const uint32_t (&w)[16], float *st, const long long *rdel,
                                              const long long *cdel, __nv_bfloat16 *out, int lane) {
   uint16_t *s2 = reinterpret_cast<uint16_t *>(st);
@@ -488,10 +545,13 @@ __device__ __forceinline__ void store_cols16(const uint32_t (&w)[16], float *st,
   }
 }
 
+enum { kAnyForm, kRuns, kAddRuns };  // the forms of output a kernel carries
+
 // A whole 32 x 32 piece (lane = row, x[j] = column j, biases added) through
 // the vector forms: the pre-activation, then the activation, then the FP32
 // and BF16 copies.  obase / tbase: the piece's base index under the primary and
 // the second map.
+template <int FORM>
 __device__ __forceinline__ void store_piece_vec(const GemmArgs &a, const long long (*del)[2][32], float (&x)[32],
                                                 float *st, int lane, long long obase, long long tbase) {
   const csrst_gemm_epilogue &ep = a.ep;
@@ -501,51 +561,50 @@ __device__ __forceinline__ void store_piece_vec(const GemmArgs &a, const long lo
     for (int j = 0; j < 32; ++j) st[lane * 33 + j] = x[j];
     __syncwarp();
   };
-  if (ep.pre) {
-    if (a.rs[0].shape == 0) {
-      store_rows32(x, st, del[0][0], del[0][1], ep.pre + obase, lane);
+  constexpr bool RUNS = FORM != kAnyForm;
+  auto store32 = [&](const RunShape &rs, float *o, auto add) {
+    constexpr bool ADD = decltype(add)::value;
+    if (rs.shape == 0) {
+      store_rows32<ADD>(x, st, del[0][0], del[0][1], o + obase, lane);
+    } else if (RUNS || rs.shape == 1) {
+      store_cols32<ADD>(x, st, del[0][0], del[0][1], o + obase, lane);
     } else {
       stage();
-      store_vec<4>(a.rs[0], st, del[0][0], del[0][1], ep.pre, obase, lane);
+      store_vec<4>(rs, st, del[0][0], del[0][1], o, obase, lane);
     }
-  }
+  };
+  if (ep.pre) store32(a.rs[0], ep.pre, std::false_type());
   if (ep.act == 1) {
 #pragma unroll
     for (int j = 0; j < 32; j += 2) gelu2(x[j], x[j + 1]);
   }
-  if (ep.out32) {
-    if (a.rs[1].shape == 0) {
-      store_rows32(x, st, del[0][0], del[0][1], ep.out32 + obase, lane);
+  if (ep.out32) store32(a.rs[1], ep.out32, std::integral_constant<bool, FORM == kAddRuns>());
+  auto store16 = [&](const RunShape &rs, void *out, const long long *rd, const long long *cd, long long base) {
+    __nv_bfloat16 *o16 = reinterpret_cast<__nv_bfloat16 *>(out);
+    if (rs.shape < 2) {
+      uint32_t w[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = bf16x2(x[2 * j], x[2 * j + 1]);
+      if (rs.shape == 0) store_rows16(w, st, rd, cd, o16 + base, lane);
+      else store_cols16(w, st, rd, cd, o16 + base, lane);
     } else {
       stage();
-      store_vec<4>(a.rs[1], st, del[0][0], del[0][1], ep.out32, obase, lane);
+      if constexpr (RUNS) store_runs<2, 8>(st, rd, cd, out, base, lane, rs.fast_j);
+      else store_vec<8>(rs, st, rd, cd, out, base, lane);
     }
-  }
-  if (ep.out16 || ep.out16t) {
-    uint32_t w[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) w[j] = bf16x2(x[2 * j], x[2 * j + 1]);
-#pragma unroll
-    for (int k = 2; k < 4; ++k) {
-      void *o = k == 2 ? ep.out16 : ep.out16t;
-      if (!o) continue;
-      const long long *rd = del[k - 2][0], *cd = del[k - 2][1];
-      const long long base = k == 2 ? obase : tbase;
-      __nv_bfloat16 *o16 = reinterpret_cast<__nv_bfloat16 *>(o);
-      if (a.rs[k].shape == 0) {
-        store_rows16(w, st, rd, cd, o16 + base, lane);
-      } else if (a.rs[k].shape == 1) {
-        store_cols16(w, st, rd, cd, o16 + base, lane);
-      } else {
-        stage();
-        store_vec<8>(a.rs[k], st, rd, cd, o, base, lane);
-      }
-    }
-  }
+  };
+  if (ep.out16) store16(a.rs[2], ep.out16, del[0][0], del[0][1], obase);
+  if (ep.out16t) store16(a.rs[3], ep.out16t, del[1][0], del[1][1], tbase);
   __syncwarp();  // the staging block is free for the next piece
 }
 
-template <int BN>
+// kRuns: every output of the launch has a vector form, the FP32 ones of shape 0 or
+// 1 and the BF16 ones 0, 1 or 2; kAddRuns: and the FP32 output is added to.  All of
+// the network's launches are one or the other; a kernel without the other forms
+// needs no spills and half the code (4096 x 256 rows, N = K = 128, GELU, BF16 output: 153
+// for 179 us with all forms in one kernel; adding to a 16384 x 128 output: 9.9 for 29 us
+// element by element).
+template <int BN, int FORM>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ GemmArgs a) {
   using G = Cfg<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -675,6 +734,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
     bool first = true;
     for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, ++lt) {
       if (lt % G::TG != g) continue;
+      const Tile tile(a, t, BN);
+      const int n0 = tile.n0, m0 = tile.m0, z = tile.z;
+      const int mrow = m0 + 32 * q, m = mrow + lane;
+      const int ncol = n0 + c * 32, n = ncol + lane;
+      const float bm = (ep.bias_m && m < a.M) ? ep.bias_m[m] : 0.0f;
       const int b = lt % G::NACC;
       int ok = 1;
       if (lane == 0)
@@ -688,11 +752,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
       tmem_wait(v);
       asm volatile("tcgen05.fence::before_thread_sync;");
       mbar_arrive(&acc_empty[b]);  // this warp's read of the accumulator is done: hand it back
-      const Tile tile(a, t, BN);
-      const int n0 = tile.n0, m0 = tile.m0, z = tile.z;
-      const int mrow = m0 + 32 * q, m = mrow + lane;
-      const int ncol = n0 + c * 32, n = ncol + lane;
-      const float bm = (ep.bias_m && m < a.M) ? ep.bias_m[m] : 0.0f;
       const uint64_t alpha = both(ep.alpha), bm2 = both(bm);
       float x[32];
       const bool whole = a.vec && mrow + 32 <= a.M && ncol + 32 <= a.N;
@@ -722,18 +781,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
         for (int j = 0; j < 32; j += 2) unpack2(add2(pack2(x[j], x[j + 1]), bm2), x[j], x[j + 1]);
       }
       if (whole) {
-        store_piece_vec(
+        store_piece_vec<FORM>(
             a, s_del, x, st, lane,
             (long long)z * ep.sb + map_part(mrow, a.md, ep.sm0, ep.sm1) + map_part(ncol, a.nd, ep.sn0, ep.sn1),
             ep.out16t ? (long long)z * ep.tb + map_part(mrow, a.tmd, ep.tm0, ep.tm1) +
                             map_part(ncol, a.tnd, ep.tn0, ep.tn1)
                       : 0);
+      } else if constexpr (FORM != kAnyForm) {
+        float y[32];  // a copy, so that x itself stays in registers
+#pragma unroll
+        for (int j = 0; j < 32; ++j) y[j] = x[j];
+        store_piece_cold(a, y, st, lane, mrow, ncol, z);
       } else {
-        const long long orow = row_part((long long)z * ep.sb, m, ep.md, ep.sm0, ep.sm1);
-        const long long trow = ep.out16t ? row_part((long long)z * ep.tb, m, ep.tmd, ep.tm0, ep.tm1) : 0;
-        const long long ocol = col_part(n, ep.nd, ep.sn0, ep.sn1);
-        const long long tcol = ep.out16t ? col_part(n, ep.tnd, ep.tn0, ep.tn1) : 0;
-        store_piece(a, x, st, lane, mrow, ncol, orow, trow, ocol, tcol);
+        store_piece(a, x, st, lane, mrow, ncol, z);
       }
     }
   }
@@ -745,15 +805,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const __grid_constant__ Ge
   }
 }
 
-// Fills the launch's vector forms; a.vec = 1 when every output has one and
-// the epilogue has no residual or accumulation (read-modify-write outputs
-// keep the element-wise path).
+// The narrowest kernel the launch can take.
+int form_of(const GemmArgs &a) {
+  const csrst_gemm_epilogue &ep = a.ep;
+  const bool runs = a.vec && !(ep.pre && a.rs[0].shape > 1) && !(ep.out32 && a.rs[1].shape > 1) &&
+                    !(ep.out16 && a.rs[2].shape > 2) && !(ep.out16t && a.rs[3].shape > 2);
+  return !runs ? kAnyForm : ep.accumulate && ep.out32 ? kAddRuns : kRuns;
+}
+
+// Fills the launch's vector forms; a.vec = 1 when every output has one, the launch
+// is kAddRuns if it adds to its output, and the epilogue has no residual (which
+// keeps the element-wise path).
 void vector_forms(GemmArgs &a, int M, int N, int batch) {
   const csrst_gemm_epilogue &ep = a.ep;
   a.vec = 0;
   const MapDesc om{ep.md, ep.nd, ep.sb, ep.sm0, ep.sm1, ep.sn0, ep.sn1};
   const MapDesc tm{ep.tmd, ep.tnd, ep.tb, ep.tm0, ep.tm1, ep.tn0, ep.tn1};
-  if (ep.res || ep.accumulate || !piece_offsets(om, a.del[0][0], a.del[0][1]) ||
+  if (ep.res || !piece_offsets(om, a.del[0][0], a.del[0][1]) ||
       (ep.out16t && !piece_offsets(tm, a.del[1][0], a.del[1][1])))
     return;
   bool ok = true;
@@ -767,6 +835,7 @@ void vector_forms(GemmArgs &a, int M, int N, int batch) {
   want(2, ep.out16, 8, 0);
   want(3, ep.out16t, 8, 1);
   a.vec = ok;
+  if (ep.accumulate && form_of(a) != kAddRuns) a.vec = 0;
 }
 
 // Polls an mbarrier wait makes before it gives up (csrst_gemm_set_wait_limit).
@@ -791,20 +860,25 @@ bool encode_operand(CUtensorMap *m, int *rank3, const __nv_bfloat16 *p, int K, l
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int BN, int FORM>
+int start_gemm(const GemmArgs &a, int dev, int grid, cudaStream_t s) {
+  using G = Cfg<BN>;
+  static unsigned long long attr = 0;  // devices the shared-memory size was set on
+  if (dev < 64 && !(attr >> dev & 1ull)) {
+    if (cudaFuncSetAttribute(k_gemm<BN, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM) != cudaSuccess)
+      return CSRST_E_CUDA;
+    attr |= 1ull << dev;
+  }
+  return launch_chained(k_gemm<BN, FORM>, dim3(grid), dim3(kThreads), G::SMEM, s, a) ? CSRST_OK : CSRST_E_CUDA;
+}
+
 template <int BN>
 int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csrst_gemm_epilogue &ep, int *err,
                 cudaStream_t s) {
-  using G = Cfg<BN>;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
                                                 cudaSuccess)
     return CSRST_E_CUDA;
-  static unsigned long long attr = 0;  // devices the shared-memory size was set on
-  if (dev < 64 && !(attr >> dev & 1ull)) {
-    if (cudaFuncSetAttribute(k_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM) != cudaSuccess)
-      return CSRST_E_CUDA;
-    attr |= 1ull << dev;
-  }
   GemmArgs a{};
   a.ep = ep;
   a.err = err;
@@ -833,13 +907,19 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   if (g1.nk && (!encode_operand(&a.map[2], &a.rank3[2], g1.A, g1.nk * kBK, M, g1.lda, g1.sA, batch, kBM, g1.amn) ||
                 !encode_operand(&a.map[3], &a.rank3[3], g1.B, g1.nk * kBK, N, g1.ldb, g1.sB, batch, BN)))
     return CSRST_E_ARG;
-  const int o_bytes = (ep.out32 || ep.res || ep.pre) ? 4 : 2;
-  a.o_mfast = rows_fast(ep.md, ep.nd, ep.sm0, ep.sm1, ep.sn0, ep.sn1, o_bytes);
-  a.t_mfast = ep.out16t ? rows_fast(ep.tmd, ep.tnd, ep.tm0, ep.tm1, ep.tn0, ep.tn1, 2) : 0;
   vector_forms(a, M, N, batch);
+  if (!a.vec || M % 32 || N % 32) {  // some pieces go element by element
+    const int o_bytes = (ep.out32 || ep.res || ep.pre) ? 4 : 2;
+    a.o_mfast = rows_fast(ep.md, ep.nd, ep.sm0, ep.sm1, ep.sn0, ep.sn1, o_bytes);
+    a.t_mfast = ep.out16t ? rows_fast(ep.tmd, ep.tnd, ep.tm0, ep.tm1, ep.tn0, ep.tn1, 2) : 0;
+  }
   a.bias4 = ep.bias && !(reinterpret_cast<uintptr_t>(ep.bias) & 15);
   const int grid = a.ntiles < sms ? a.ntiles : sms;
-  return launch_chained(k_gemm<BN>, dim3(grid), dim3(kThreads), G::SMEM, s, a) ? CSRST_OK : CSRST_E_CUDA;
+switch (form_of(a)) {
+    case kRuns: return start_gemm<BN, kRuns>(a, dev, grid, s);
+    case kAddRuns: return start_gemm<BN, kAddRuns>(a, dev, grid, s);
+    default: return start_gemm<BN, kAnyForm>(a, dev, grid, s);
+  }
 }
 
 bool seg_ok(const void *A, long long lda, long long sa, const void *B, long long ldb, long long sb, int K) {

@@ -93,17 +93,16 @@ inline bool bases_aligned(const MapDesc &d, int M, int N, int batch, const void 
 inline RunShape run_shape(const long long *rdel, const long long *cdel, int L) {
   for (int S = 0; S < 4; ++S) {
     const int ri = S == 0 ? 1 : S == 1 ? L : S == 2 ? L / 2 : 2, rj = S == 0 ? L : S == 1 ? 1 : S == 2 ? 2 : L / 2;
-    bool ok = true;
-    for (int oi = 0; oi < 32 && ok; oi += ri)
-      for (int oj = 0; oj < 32 && ok; oj += rj) {
-        const long long o = rdel[oi] + cdel[oj];
-        ok = mod_pos(o, L) == 0;
-        for (int t = 0; t < L && ok; ++t) {
-          const int i = oi + (S == 0 ? 0 : S == 1 ? t : S == 2 ? t / 2 : t % 2);
-          const int j = oj + (S == 0 ? t : S == 1 ? 0 : S == 2 ? t % 2 : t / 2);
-          ok = rdel[i] + cdel[j] == o + t;
-        }
-      }
+    // the index is a sum of a row and a column part, so each is checked by itself:
+    // along a run a row step advances by tr and a column step by tc, and every
+    // run starts on a multiple of L
+    const int tr = S == 2 ? 2 : 1, tc = S == 3 ? 2 : 1;
+    bool ok = mod_pos(rdel[0] + cdel[0], L) == 0;
+    for (int i = 0; i < 32 && ok; ++i) {
+      const int oi = i - i % ri, oj = i - i % rj;
+      ok = rdel[i] == rdel[oi] + (long long)(i % ri) * tr && cdel[i] == cdel[oj] + (long long)(i % rj) * tc &&
+           mod_pos(rdel[oi] - rdel[0], L) == 0 && mod_pos(cdel[oj] - cdel[0], L) == 0;
+    }
     if (!ok) continue;
     const int ni = 32 / ri, nj = 32 / rj;
     int best = 1 << 30, fast = 1;

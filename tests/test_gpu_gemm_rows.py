@@ -53,3 +53,32 @@ def test_row_and_column_stores(gpu_lib, M, N, batch, bias_off, row_bias):
     assert torch.equal(o16t.cpu()[..., :M].transpose(1, 2), o16.cpu()[..., :N])
     assert bool((pre[..., N:] == 9).all() and (o32[..., N:] == 9).all() and (o16[..., N:] == 9).all())
     assert bool((o16t[..., M:] == 9).all())
+
+
+@pytest.mark.parametrize("M,N,batch", [(32, 32, 1), (33, 48, 2), (128, 128, 3), (250, 160, 2)])
+@pytest.mark.parametrize("columns", [False, True])
+def test_adding_to_the_output(gpu_lib, M, N, batch, columns):
+    """accumulate through row and column runs and the ragged edge, with a BF16 copy of the
+    product alone: the FP32 output is the one addition of the old value, exactly."""
+    import torch
+    from csrst_b200.tensor import check_errors, gemm
+    K, Mp = 64, (M + 7) // 8 * 8
+    g = torch.Generator().manual_seed(M + N)
+    a = torch.randn(batch, M, K, generator=g).to(torch.bfloat16).cuda()
+    b = torch.randn(batch, N, K, generator=g).to(torch.bfloat16).cuda()
+    shape = (batch, N, Mp) if columns else (batch, M, N)
+    old = torch.randn(shape, generator=g).cuda()
+    omap = dict(md=1, nd=1, sm0=1, sm1=0, sn0=Mp, sn1=0) if columns else None
+    sb = shape[1] * shape[2]
+    once, twice = torch.zeros(shape, device="cuda"), old.clone()
+    o16 = torch.zeros(shape, dtype=torch.bfloat16, device="cuda")
+    kw = dict(batch=batch, stride_a=M * K, stride_b=N * K, omap=omap, sb=sb)
+    gemm(a, b, M, N, K, out32=once, **kw)
+    gemm(a, b, M, N, K, out32=twice, out16=o16, accumulate=True, **kw)
+    torch.cuda.synchronize()
+    check_errors()
+    r = a.double() @ b.double().transpose(1, 2)
+    got = once.transpose(1, 2)[:, :M] if columns else once
+    assert float((got.double() - r).abs().max()) <= 1e-4 * float(r.abs().max())
+    assert torch.equal(twice, old + once)
+    assert torch.equal(o16, once.to(torch.bfloat16))
