@@ -9,6 +9,7 @@
 // step 1754 us, where the same launches replayed as a graph took 141 and 972 us.  From
 // here a launch costs its tensor maps and the launch itself: 163 and 1155 us with
 // the kernels as they were then.  Nothing is kept between calls: every pointer comes in with the call.
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/csrst.h"
@@ -42,15 +43,54 @@ csrst_gemm_epilogue epilogue(const Map &m, long long sb = 0) {
 
 // The network with the offsets of its parameters in the flat buffer, and the
 // first error of the sequence (later launches are then left out).
+//
+// A training step's weight gradients, bias sums and the transposes they need lie off
+// the chain of activations and gradients, and most launches fill a part of the chip
+// only, so they go to the side stream: aside(f) runs f's launches there after
+// what the main stream holds so far, rejoin() makes the main stream wait for all
+// of them.  A buffer that work aside reads is written again only after a rejoin, and
+// the calls end with one, whatever happened in between.  (`part` and `cpart` are
+// used aside, or after the last rejoin.)  64 members: 556 us a step, 630 on one
+// stream.
 struct Seq {
   const csrst_fno &f;
   int *err;
   void *s;
   int rc = CSRST_OK;
   long long w, m, R, B;
+  cudaStream_t main, side;
+  cudaEvent_t out = nullptr, back = nullptr;
 
-  Seq(const csrst_fno &net, int *e, void *stream)
-      : f(net), err(e), s(stream), w(net.width), m(net.modes), R((long long)net.batch * kBins), B(net.batch) {}
+  Seq(const csrst_fno &net, int *e, void *stream, bool two)
+      : f(net), err(e), s(stream), w(net.width), m(net.modes), R((long long)net.batch * kBins), B(net.batch),
+        main(static_cast<cudaStream_t>(stream)), side(two ? static_cast<cudaStream_t>(net.side) : nullptr) {
+    if (side && (cudaEventCreateWithFlags(&out, cudaEventDisableTiming) != cudaSuccess ||
+                 cudaEventCreateWithFlags(&back, cudaEventDisableTiming) != cudaSuccess))
+      rc = CSRST_E_CUDA;
+  }
+  ~Seq() {
+    if (out) cudaEventDestroy(out);
+    if (back) cudaEventDestroy(back);
+  }
+  Seq(const Seq &) = delete;
+
+  void cuda(cudaError_t e) { ck(e == cudaSuccess ? CSRST_OK : CSRST_E_CUDA); }
+  template <class F>
+  void aside(F launches) {
+    if (!ok()) return;
+    if (side) {
+      cuda(cudaEventRecord(out, main));
+      cuda(cudaStreamWaitEvent(side, out, 0));
+      s = side;
+    }
+    launches();
+    s = main;
+  }
+  void rejoin() {  // also after an error
+    if (!side || !out || !back) return;
+    cuda(cudaEventRecord(back, side));
+    cuda(cudaStreamWaitEvent(main, back, 0));
+  }
 
   void ck(int r) {
     if (rc == CSRST_OK) rc = r;
@@ -122,14 +162,14 @@ void forward(Seq &q, const void *X16, float *out) {
   for (int l = 0; l < f.layers; ++l) {
     const int i = tr ? l : l & 1, o = tr ? l + 1 : (l + 1) & 1;
     const bool act = l < f.layers - 1;
-    if (tr) q.transpose16(f.V16[i], f.Vg16[i], 1, R, w, R);
+    if (tr) q.aside([&] { q.transpose16(f.V16[i], f.Vg16[i], 1, R, w, R); });
     // forward DFT over the bins, per member b: rows c of V[b] read MN-major -> U[k][b][2c + ri]
     ep = epilogue({1, 2, 2, 0, 2 * w * B, 1}, 2 * w);
     ep.out16 = f.U16;
     if (q.ok())
       q.ck(csrst_gemm_bf16_ex(f.V16[i], w, kBins * w, 1, f.F16, kBins, 0, (int)w, (int)(2 * m), kBins, (int)B, &ep,
                               q.err, q.s));
-    if (tr) q.transpose16(f.U16, f.Ut16[l], m, B, 2 * w, B);
+    if (tr) q.aside([&] { q.transpose16(f.U16, f.Ut16[l], m, B, 2 * w, B); });
     // mode mixing: per mode k, Z[b][2o + p] = sum U[b][2c + q] Mk[2o + p][2c + q]
     ep = epilogue(rows_of(2 * w), 2 * w * B);
     ep.out16 = f.Z16;
@@ -144,9 +184,10 @@ void forward(Seq &q, const void *X16, float *out) {
     if (q.ok())
       q.ck(csrst_gemm_bf16_dual(f.Zp16, 2 * m, 2 * m * w, f.G16, 2 * m, 0, (int)(2 * m), q.p16(q.oW(l)), w, 0,
                                 f.V16[i], w, kBins * w, (int)w, (int)w, kBins, (int)B, &ep, q.err, q.s));
+    if (tr) q.rejoin();  // U16 is written again in the next layer
   }
   void *V = f.V16[tr ? f.layers : f.layers & 1];
-  if (tr) q.transpose16(V, f.Vg16[f.layers], 1, R, w, R);
+  if (tr) q.aside([&] { q.transpose16(V, f.Vg16[f.layers], 1, R, w, R); });
   ep = epilogue(rows_of(w));
   ep.bias = q.p32(q.oq1());
   ep.act = 1;
@@ -163,6 +204,7 @@ void forward(Seq &q, const void *X16, float *out) {
   ep.bias = q.p32(q.oq2());
   ep.out32 = out;
   q.gemm(f.A1_16, q.p16(q.oQ2()), R, f.nout, w, ep);
+  if (tr) q.rejoin();
 }
 
 void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
@@ -173,34 +215,44 @@ void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
   if (q.ok())
     q.ck(csrst_nn_mse(f.out, T, Wt, R * nout, f.dOut, (int)nout, 64, 1, f.lpart, f.loss, q.s));
   if (q.ok()) q.ck(csrst::nn_backward_rows(f.dOut, nullptr, nullptr, f.dOut16, f.dOutT16, (int)R, 64, q.s));
-  q.wgrad(f.dOutT16, f.A1t16, nout, w, q.g32(q.oQ2()));
-  q.colsum(f.dOut, R, 64, q.g32(q.oq2()));  // q2 and the padding after it
+  q.aside([&] {
+    q.wgrad(f.dOutT16, f.A1t16, nout, w, q.g32(q.oQ2()));
+    q.colsum(f.dOut, R, 64, q.g32(q.oq2()));  // q2 and the padding after it
+    q.transpose16(X16, f.Xt16, 1, R, kFeat, R);
+  });
   ep = epilogue(rows_of(w));
   ep.out32 = f.dA1;
   q.gemm(f.dOut16, f.Q2T16, R, w, 64, ep);
   q.activation_bwd(f.dA1, f.A1pre, f.dH);
-  q.wgrad(f.dHt16, f.Vg16[f.layers], w, w, q.g32(q.oQ1()));
-  q.colsum(f.dH, R, w, q.g32(q.oq1()));
+  q.aside([&] {
+    q.wgrad(f.dHt16, f.Vg16[f.layers], w, w, q.g32(q.oQ1()));
+    q.colsum(f.dH, R, w, q.g32(q.oq1()));
+  });
   ep.out32 = f.dV;
   q.gemm(f.dH16, f.Q1T16, R, w, w, ep);
   float *dV = f.dV, *dVn = f.dVn;
   for (int l = f.layers - 1; l >= 0; --l) {
     const bool act = l < f.layers - 1;
     const float *dH = act ? f.dH : dV;
+    q.rejoin();  // dH, dH16, dHt16, dZt16 and the gradient before last are free
     q.activation_bwd(dV, act ? f.Hfull[l] : nullptr, act ? f.dH : nullptr);
-    q.wgrad(f.dHt16, f.Vg16[l], w, w, q.g32(q.oW(l)));
-    q.colsum(dH, R, w, q.g32(q.ob(l)));
+    q.aside([&] {
+      q.wgrad(f.dHt16, f.Vg16[l], w, w, q.g32(q.oW(l)));
+      q.colsum(dH, R, w, q.g32(q.ob(l)));
+    });
     // adjoint of the inverse DFT: dZ[k][(o, ri)][b] = sum_n dH[b][n][o] G[n][2k + ri] (rows (o, b) of dH^T)
     ep = epilogue({(int)B, 2, 2 * B, 1, 2 * w * B, B});
     ep.out16 = f.dZt16;
     q.gemm(f.dHt16, f.GT16, w * B, 2 * m, kBins, ep);
     q.transpose16(f.dZt16, f.dZ16, m, 2 * w, B, 2 * w);
     // mode-mixing weights: dMk[k] = dZ_k^T U_k, then back to (dWr, dWi)
-    ep = epilogue(rows_of(2 * w), 4 * w * w);
-    ep.out32 = f.dMk;
-    q.gemm_batched(f.dZt16, B, 2 * w * B, f.Ut16[l], B, 2 * w * B, 2 * w, 2 * w, B, m, ep);
-    if (q.ok())
-      q.ck(csrst_nn_spectral_unpack(f.dMk, (int)m, (int)w, q.g32(q.oWr(l)), q.g32(q.oWi(l)), q.s));
+    q.aside([&] {
+      csrst_gemm_epilogue e = epilogue(rows_of(2 * w), 4 * w * w);
+      e.out32 = f.dMk;
+      q.gemm_batched(f.dZt16, B, 2 * w * B, f.Ut16[l], B, 2 * w * B, 2 * w, 2 * w, B, m, e);
+      if (q.ok())
+        q.ck(csrst_nn_spectral_unpack(f.dMk, (int)m, (int)w, q.g32(q.oWr(l)), q.g32(q.oWi(l)), q.s));
+    });
     // dU_k = dZ_k Mk -> dSk[k][b][2c + q] -> dS[(b, c)][2k + q]
     ep = epilogue(rows_of(2 * w), 2 * w * B);
     ep.out16 = f.dSk16;
@@ -218,8 +270,8 @@ void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
     dV = dVn;
     dVn = t;
   }
+  q.rejoin();
   q.activation_bwd(dV, nullptr, nullptr);
-  q.transpose16(X16, f.Xt16, 1, R, kFeat, R);
   q.wgrad(f.dHt16, f.Xt16, w, kFeat, q.g32(q.oP()));
   q.colsum(dV, R, w, q.g32(q.op()));
 }
@@ -230,22 +282,22 @@ extern "C" {
 
 int csrst_fno_forward(const csrst_fno *f, const void *X16, float *out, int *err, void *stream) {
   if (!valid(f, err) || !X16 || !out) return CSRST_E_ARG;
-  Seq q(*f, err, stream);
-  forward(q, X16, out);
+  Seq q(*f, err, stream, f->train);
+  if (q.ok()) forward(q, X16, out);
   return q.rc;
 }
 
 int csrst_fno_backward(const csrst_fno *f, const void *X16, const float *T, const float *Wt, int *err, void *stream) {
   if (!valid(f, err) || !f->train || !f->g || !X16 || !T) return CSRST_E_ARG;
-  Seq q(*f, err, stream);
-  backward(q, X16, T, Wt);
+  Seq q(*f, err, stream, true);
+  if (q.ok()) backward(q, X16, T, Wt);
   return q.rc;
 }
 
 int csrst_fno_refresh(const csrst_fno *f, long long n, void *stream) {
   int none = 0;
   if (!valid(f, &none) || n <= 0) return CSRST_E_ARG;
-  Seq q(*f, &none, stream);
+  Seq q(*f, &none, stream, false);
   const long long w = q.w;
   q.cast(f->w, f->w16, n);
   for (int l = 0; l < f->layers; ++l) {

@@ -84,7 +84,7 @@ class _Net(C.Structure):
                     "w", "g", "w16", "WT16", "Mk16", "MkT16", "Q1T16", "Q2T16", "F16", "FT16", "G16", "GT16", "V16",
                     "U16", "Z16", "Zp16", "A1_16", "out", "Vg16", "Ut16", "Hfull", "A1pre", "A1t16", "Xt16", "dOut",
                     "dOut16", "dOutT16", "dA1", "dH", "dH16", "dHt16", "dV", "dVn", "dZ16", "dZt16", "dSk16", "dS16",
-                    "dMk", "part", "cpart", "lpart", "loss")])
+                    "dMk", "part", "cpart", "lpart", "loss", "side")])
 
 
 def _ptrs(ts):
@@ -146,6 +146,15 @@ class _Buffers:
         self.cpart = torch.empty(max(B * max(w, 64), ((R // KSPLIT + 255) // 256) * w * max(w, NFEAT)), **f32)
         self.lpart = torch.empty(256, dtype=torch.float64, device=dev)
         self.loss = torch.zeros(1, dtype=torch.float64, device=dev)
+        self.side = torch.cuda.Stream(dev)  # joined to the caller's stream within each call
+
+    def __getstate__(self):   # a copy gets a side stream of its own
+        return {k: v for k, v in vars(self).items() if k != "side"}
+
+    def __setstate__(self, d):
+        vars(self).update(d)
+        if self.train:
+            self.side = torch.cuda.Stream(self.loss.device)
 
 
 class FNO:
@@ -227,6 +236,8 @@ class FNO:
                     v = _ptrs(v)
                     n.keep.append(v)
                     setattr(n, k, C.addressof(v))
+                elif k == "side":
+                    n.side = v.cuda_stream
                 elif k != "train":
                     setattr(n, k, v.data_ptr())
         return n

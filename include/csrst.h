@@ -331,6 +331,7 @@ typedef struct {
   float *dMk;                                        /* [modes][2 width][2 width] */
   float *part, *cpart;                               /* partial products, column-sum scratch */
   double *lpart, *loss;                              /* 256 doubles of scratch, the loss */
+  void *side;                                        /* a second stream for work off the critical path, or NULL */
 } csrst_fno;
 /* out [R][nout] (FP32) for X16 [R][64] (BF16); *err as for the GEMM */
 int csrst_fno_forward(const csrst_fno *f, const void *X16, float *out, int *err, void *stream);
