@@ -227,6 +227,7 @@ struct csrst_ensemble {
   int epar = 0;              // plane-set swaps of the fused sweep since the tables were built, mod 2
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step, per parity
   bool holds = false;        // the members' ens_refs count this ensemble
+  void *derr = nullptr;      // csrst_ensemble_sync: the members' window states and their errors
   std::string err;
 };
 
@@ -1218,8 +1219,7 @@ int csrst_get_particles(csrst_handle *h, double *x, double *y, double *px, doubl
     double *dst[4] = {x, y, px, py};
     for (int k = 0; k < 4; ++k)
       if (dst[k]) CK(cudaMemcpyAsync(dst[k], src[k], (size_t)h->n * sizeof(double), cudaMemcpyDeviceToHost, h->s));
-    CK(cudaStreamSynchronize(h->s));
-    return check_err(h);
+    return check_err(h);  // (its copy follows these, and it waits)
   }
   materialise(h);
   const size_t nb = (size_t)h->n * sizeof(double);
@@ -1227,7 +1227,6 @@ int csrst_get_particles(csrst_handle *h, double *x, double *y, double *px, doubl
   if (y) CK(cudaMemcpyAsync(y, h->y, nb, cudaMemcpyDeviceToHost, h->s));
   if (px) CK(cudaMemcpyAsync(px, h->px, nb, cudaMemcpyDeviceToHost, h->s));
   if (py) CK(cudaMemcpyAsync(py, h->py, nb, cudaMemcpyDeviceToHost, h->s));
-  CK(cudaStreamSynchronize(h->s));
   return check_err(h);
 }
 
@@ -1459,10 +1458,10 @@ int csrst_diag_wake(csrst_handle *h, double *out, int n) {
   double *d = nullptr;
   CK(cudaMallocAsync(&d, (size_t)n * sizeof(double), h->s));
   if (h->fp32)
-    launch_wake(h->ws, wplane32(h, 0).p, wplane32(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, d,
+    launch_wake(h->ws, wplane32(h, 0).p, wplane32(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, d, nullptr,
                 h->s);
   else
-    launch_wake(h->ws, wplane(h, 0).p, wplane(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, d, h->s);
+    launch_wake(h->ws, wplane(h, 0).p, wplane(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, d, nullptr, h->s);
   CK(cudaMemcpyAsync(out, d, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, h->s));
   CK(cudaFreeAsync(d, h->s));
   CK(cudaStreamSynchronize(h->s));
@@ -1527,11 +1526,11 @@ int csrst_diag_wake_async(csrst_handle *h, double *out_dev, int n, double *meta_
   moments_async(h);
   if (h->fp32)
     launch_wake(h->ws, wplane32(h, 0).p, wplane32(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, out_dev,
-                h->s);
+                meta_dev, h->s);
   else
-    launch_wake(h->ws, wplane(h, 0).p, wplane(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, out_dev, h->s);
-  CK(cudaMemcpyAsync(meta_dev, &h->ws->mo0, 2 * sizeof(double), cudaMemcpyDeviceToDevice, h->s));
-  CK(cudaMemcpyAsync(meta_dev + 2, h->dmean, 2 * sizeof(double), cudaMemcpyDeviceToDevice, h->s));
+    launch_wake(h->ws, wplane(h, 0).p, wplane(h, 1).p, h->wpitch, h->L0, h->b.hr0, h->b.hr1, h->dmean, out_dev,
+                meta_dev, h->s);
+  CK(cudaGetLastError());
   return CSRST_OK;
 }
 
@@ -1955,6 +1954,7 @@ int csrst_ensemble_destroy(csrst_ensemble *e) {
   if (e->holds)
     for (csrst_handle *h : e->mem) --h->ens_refs;
   ensemble_free_tables(e);
+  cudaFree(e->derr);
   if (e->done) cudaEventDestroy(e->done);
   if (e->fork) cudaEventDestroy(e->fork);
   if (e->s) cudaStreamDestroy(e->s);
@@ -1996,11 +1996,37 @@ int csrst_ensemble_step(csrst_ensemble *e, int nsteps) {
   return ensemble_release(e);
 }
 
+// All members' streams have ended and no member has a sticky error (false also
+// where that cannot be told here: the caller then asks each member).
+static bool ensemble_clean(csrst_ensemble *e) {
+  std::vector<const WinState *> ws(e->m);
+  for (int k = 0; k < e->m; ++k) {
+    ws[k] = e->mem[k]->ws;
+    if (!ws[k] || cudaStreamSynchronize(e->mem[k]->s) != cudaSuccess) return false;
+  }
+  if (!e->derr && cudaMalloc(&e->derr, (size_t)e->m * (sizeof(WinState *) + sizeof(int))) != cudaSuccess) {
+    e->derr = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  const WinState **tab = static_cast<const WinState **>(e->derr);
+  int *out = reinterpret_cast<int *>(tab + e->m);
+  std::vector<int> err(e->m, 1);
+  if (cudaMemcpyAsync(tab, ws.data(), ws.size() * sizeof(ws[0]), cudaMemcpyHostToDevice, e->s) != cudaSuccess)
+    return false;
+  launch_member_errors(tab, e->m, out, e->s);
+  if (cudaMemcpyAsync(err.data(), out, err.size() * sizeof(int), cudaMemcpyDeviceToHost, e->s) != cudaSuccess ||
+      cudaStreamSynchronize(e->s) != cudaSuccess || cudaPeekAtLastError() != cudaSuccess)
+    return false;
+  return std::all_of(err.begin(), err.end(), [](int v) { return v == 0; });
+}
+
 // Sticky device errors of all members: the first member with one, or 0.
 int csrst_ensemble_sync(csrst_ensemble *e, int *bad_member) {
   if (!e) return CSRST_E_ARG;
   if (bad_member) *bad_member = -1;
   if (cudaStreamSynchronize(e->s) != cudaSuccess) return efail(e, CSRST_E_CUDA, "ensemble stream");
+  if (ensemble_clean(e)) return CSRST_OK;
   for (int k = 0; k < e->m; ++k) {
     const int rc = csrst_sync(e->mem[k]);
     if (rc) {

@@ -245,7 +245,8 @@ void launch_field_energy(const T *Ex, const T *Ey, const T *Hx, const T *Hy, int
 size_t moments_scratch_doubles();
 template <class T>
 void launch_wake(const WinState *ws, const T *mEx, const T *mEy, int wpitch, int L0, double h0, double h1,
-                 const double *mean, double *out, cudaStream_t s);
+                 const double *mean, double *out, double *meta, cudaStream_t s);  // meta (may be NULL): window origin and bunch mean
+void launch_member_errors(const WinState *const *ws, int m, int *out, cudaStream_t s);
 void launch_charge_diff(int order, const double *ox, const double *oy, const double *x, const double *y,
                         const double *q, long long n, double org0, double org1, double h0, double h1,
                         int i0, int j0, int ni, int nj, unsigned long long *acc, double scale,
