@@ -103,10 +103,10 @@ def peaks(bf16=False):
 # The launches of one time step per kernel group (order 1 = TSC), as the
 # profile launch lists name them.
 STEP_LAUNCHES = {
-    ("push", "fp32", 1): {"k_push32<1, 0>": 1, "k_push32<1, 1>": 1, "k_prep32": 1, "k_after32": 2},
-    ("yee", "fp32", 1): {"k_yee_tiles<float>": 1, "k_yee_fixup<float>": 1, "k_window_ey<float>": 1},
-    ("push", "fp64", 1): {"k_push<1>": 2, "k_push_prep": 2, "k_push_post": 2, "k_global_bounds": 2},
-    ("yee", "fp64", 1): {"k_yee_tiles<double>": 1, "k_yee_fixup<double>": 1, "k_window_ey<double>": 1},
+    ("push", "fp32", 1): {"k_push32<1, 0>": 1, "k_push32<1, 1>": 1},
+    ("yee", "fp32", 1): {"k_yee_tiles<float>": 1, "k_yee_fixup<float>": 1, "k_step_tail<float>": 1},
+    ("push", "fp64", 1): {"k_push<1, 0>": 1, "k_push<1, 1>": 1},
+    ("yee", "fp64", 1): {"k_yee_tiles<double>": 1, "k_yee_fixup<double>": 1, "k_step_tail<double>": 1},
 }
 LAUNCH_LISTS = {"fp32": "profiles/c2_tsc_fp32_step_launches.txt", "fp64": "profiles/c2_tsc_fp64_step_launches.txt"}
 
@@ -406,7 +406,10 @@ def run_ensemble(args, rank, members=64, ms=None, fields=True):
     for sm in sims:
         sm.close()
     out["fp32_batched"] = {"value": round(total * K / (msb * 1e-3), 1), "ms_per_step": round(msb / K, 3),
-                           "launches_per_step": 4 * 2 + 2 * 4 + 2 + 1,
+                           # per part: both pushes (set-up, one launch a shape order, bookkeeping), then tiles,
+                           # fix-ups and tail, or nine sub-step launches
+                           "launches_per_step": int(best[3]) * (2 * (2 + len({c.shape_order for c, _ in ms})) +
+                                                                (9 if best[1] else 3)),
                            "tuned_shape": {"push_ctas": int(best[0]), "tile": [int(best[1]), int(best[2])],
                                            "parts": int(best[3])},
                            "tuning_table_ms": [[int(r[0]), int(r[1]), int(r[2]), int(r[3]), round(r[4], 3)]
@@ -523,7 +526,7 @@ def run_surrogate(args):
     torch.cuda.synchronize()
     net.check()
     out["training"] = {"batch": B, "ms_per_step": round(a.elapsed_time(b) / 200, 4),
-                       "library_calls_per_step": 106,
+                       "library_calls_per_step": 5,
                        "what": "forward, hand-written backward and Adam, captured as one CUDA graph"}
     del g
     # the PIC it replaces: 256 data-set cases as one ensemble
@@ -634,11 +637,9 @@ def run_b200(args, world, rank, local):
     if other in runs:
         out[other] = summary(other)
         out[f"{head}_over_{other}"] = round(hs["value"] / out[other]["value"], 3)
-    # launches per FP32 step: the first push (prep, push, closing kernel that
-    # also sets up the second), the second push (push, closing kernel), the
-    # fused field sweep (tiles, window fix-up), the window's Ey, and the move
-    # (two copy stages, finish)
-    out["gpu_launches"] = args.steps * (3 + 2 + 2 + 1 + 3)
+    # launches per step: two pushes (with their bookkeeping), the fused field
+    # sweep (tiles, window fix-up) and the step's tail (window Ey, move, next set-up)
+    out["gpu_launches"] = args.steps * (2 + 2 + 1)
     if rank == 0 and not args.no_compare:
         out["accuracy_fp32_vs_fp64"] = accuracy(cfg, spec, bunch)
     if not args.no_ensemble:

@@ -170,7 +170,9 @@ int csrst_step(csrst_handle *h, int nsteps);
  * events between its kernel groups; waits for it and returns the device
  * times in ms4 [ms]: both pushes, the field work (the fused sweep, or the
  * four sub-steps with their exchanges, and the window's Ey), the window move,
- * and the whole step. */
+ * and the whole step.  In the fused step the second push runs beside the
+ * sweep's tiles, so the groups overlap and their sum is above the whole; where the
+ * window's Ey and its move are one launch, it counts as field work and the move is 0. */
 int csrst_step_timed(csrst_handle *h, double *ms4);
 /* Polls a fused-sweep tile makes in its staging wait (the TMA copies of its
  * fields) before it gives up, writes nothing and reports CSRST_E_STAGING at
@@ -206,9 +208,9 @@ int csrst_ensemble_step(csrst_ensemble *e, int nsteps);
 /* Waits for the ensemble; returns the first member's sticky error (its index in *bad_member). */
 int csrst_ensemble_sync(csrst_ensemble *e, int *bad_member);
 /* Launch shapes: CTAs of the batched push (0 = two per SM), the field path
- * (tx = ty = 0: the fused static sweep, all members' tiles and window
- * fix-ups from one work queue in one persistent launch per step, the
- * default; else one launch per sub-step with static-sweep tiles of tx x ty,
+ * (tx = ty = 0: the fused static sweep, all members' tiles from one work
+ * queue in one persistent launch per step beside a launch of their window
+ * fix-ups, the default; else one launch per sub-step with static-sweep tiles of tx x ty,
  * tx * ty = 256) and the number of parts the members are split into, which
  * step side by side on their own streams.  Results do not depend on them. */
 int csrst_ensemble_set_shape(csrst_ensemble *e, int push_ctas, int tx, int ty, int parts);
