@@ -82,7 +82,7 @@ struct TileAcc {
   }
 
   // Re-bases the warp's tile on the start cell of a middle lane of those that
-  // have a particle (has) in this round: they are sorted along x, so the tile
+  // have a particle (has) in this pass: they are sorted along x, so the tile
   // then reaches as far to either side.
   template <bool SHARED>
   __device__ __forceinline__ void rebase(bool has, int ci, int cj, unsigned long long *dst, int L0, int L1) {

@@ -390,14 +390,13 @@ __device__ __noinline__ void store_piece_cold(const GemmArgs &a, float (&x)[32],
   store_piece(a, x, st, lane, mrow, ncol, z);
 }
 
-// Row and column offsets of element t of a run of shape S, and the run's
-// extent in rows (RI) and columns (RJ).
+// Row and column offsets of element t of a run of shape S (2 or 3: pairs), and
+// the run's extent in rows (RI) and columns (RJ).
 template <int S, int L>
 struct Run {
-  static constexpr int RI = S == 0 ? 1 : S == 1 ? L : S == 2 ? L / 2 : 2;
-  static constexpr int RJ = S == 0 ? L : S == 1 ? 1 : S == 2 ? 2 : L / 2;
-  static __device__ __forceinline__ int di(int t) { return S == 0 ? 0 : S == 1 ? t : S == 2 ? t >> 1 : t & 1; }
-  static __device__ __forceinline__ int dj(int t) { return S == 0 ? t : S == 1 ? 0 : S == 2 ? t & 1 : t >> 1; }
+  static constexpr int RI = S == 2 ? L / 2 : 2, RJ = S == 2 ? 2 : L / 2;
+  static __device__ __forceinline__ int di(int t) { return S == 2 ? t >> 1 : t & 1; }
+  static __device__ __forceinline__ int dj(int t) { return S == 2 ? t & 1 : t >> 1; }
 };
 
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
@@ -432,12 +431,8 @@ __device__ __forceinline__ void store_runs(const float *st, const long long *rde
 template <int L>
 __device__ __forceinline__ void store_vec(const RunShape &rs, const float *st, const long long *rdel,
                                           const long long *cdel, void *out, long long base, int lane) {
-  switch (rs.shape) {
-    case 0: store_runs<0, L>(st, rdel, cdel, out, base, lane, rs.fast_j); break;
-    case 1: store_runs<1, L>(st, rdel, cdel, out, base, lane, rs.fast_j); break;
-    case 2: store_runs<2, L>(st, rdel, cdel, out, base, lane, rs.fast_j); break;
-    default: store_runs<3, L>(st, rdel, cdel, out, base, lane, rs.fast_j); break;
-  }
+  if (rs.shape == 2) store_runs<2, L>(st, rdel, cdel, out, base, lane, rs.fast_j);
+  else store_runs<3, L>(st, rdel, cdel, out, base, lane, rs.fast_j);
 }
 
 // *at(k) += of(k) for a lane's eight runs, the reads four at a time.
