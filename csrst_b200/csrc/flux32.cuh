@@ -65,11 +65,11 @@ struct Flux32Shape;
 // S: charge stencil width; OFF: first stencil vertex relative to the base
 // index; DUAL: the path integral splits at dual-cell (half-integer) borders.
 template <>
-struct Flux32Shape<0> { static constexpr int S = 2, OFF = 0, CEN = 0; static constexpr bool DUAL = false; };
+struct Flux32Shape<0> { static constexpr int S = 2, OFF = 0; static constexpr bool DUAL = false; };
 template <>
-struct Flux32Shape<1> { static constexpr int S = 3, OFF = -1, CEN = 1; static constexpr bool DUAL = true; };
+struct Flux32Shape<1> { static constexpr int S = 3, OFF = -1; static constexpr bool DUAL = true; };
 template <>
-struct Flux32Shape<2> { static constexpr int S = 4, OFF = -1, CEN = 1; static constexpr bool DUAL = false; };
+struct Flux32Shape<2> { static constexpr int S = 4, OFF = -1; static constexpr bool DUAL = false; };
 
 // Arithmetic with one rounding per operation, whatever contraction the
 // including file is compiled with: the compact and the general form of the
@@ -112,18 +112,21 @@ __device__ __forceinline__ long long round_product(double T, double w) {
 }
 
 // Base index of the offset o relative to its cell: floor(o), or floor(o + 1/2)
-// for the quadratic shape, exactly (o + 0.5f may round up to the next integer).
+// for the quadratic shape, exactly.  (o + 0.5f rounds 0.5 - 2^-25 up to 1: a form
+// chosen by that sum put such an end point's charge one row or column off.)
 template <int ORDER>
-__device__ __forceinline__ int exact_base(float o) {
+__device__ __forceinline__ int base_index(float o) {
   const float f = floorf(o);
   return (int)f + (ORDER == 1 && f_sub(o, f) >= 0.5f ? 1 : 0);
 }
 
-// Base indices of a move's end points (old-cell relative), for choosing the
-// deposit's form before running it.
+// Whether a move of charge K takes the compact form of the deposit
+// (flux_compact): it keeps its y base index, advances its x base index by 0 or 1,
+// and |K| < kRoundMax.  The general form gives the same integers for it.
 template <int ORDER>
-__device__ __forceinline__ int base_index(float o) {
-  return (int)floorf(ORDER == 1 ? f_add(o, 0.5f) : o);
+__device__ __forceinline__ bool compact_form(float a0, float a1, int dc0, int dc1, float b0, float b1, double K) {
+  return (unsigned)(dc0 + base_index<ORDER>(b0) - base_index<ORDER>(a0)) <= 1u &&
+         dc1 + base_index<ORDER>(b1) == base_index<ORDER>(a1) && fabs(K) < kRoundMax;
 }
 
 // Base index (relative to the cell of the offset) and 1D charge weights of
@@ -132,7 +135,7 @@ __device__ __forceinline__ int base_index(float o) {
 // .cpp:408-441 (cubic), in FP64 on the exact offset.
 template <int ORDER>
 __device__ __forceinline__ int charge_weights(float o, double *w) {
-  const int f = exact_base<ORDER>(o);
+  const int f = base_index<ORDER>(o);
   const double a = d_sub((double)o, (double)(float)f);
   if (ORDER == 0) {
     w[0] = d_sub(1.0, a); w[1] = a;
@@ -310,9 +313,8 @@ __device__ __forceinline__ float displacement(int dc, float b, float a) {
   return (float)d_add((double)dc, d_sub((double)b, (double)a));
 }
 
-// The compact form of the deposit below, for moves that keep their y base
-// index and advance their x base index by 0 or 1 (a bunch moving along +x at
-// CFL <= 1, nearly every particle) and |K| < kRoundMax: the stencil box has
+// The compact form of the deposit below, for the moves of compact_form (a bunch
+// moving along +x at CFL <= 1, nearly every particle): the stencil box has
 // S + 1 columns and S rows, start weights unshifted, and every index is a
 // compile-time constant.  The second segment (from the x crossing on) is
 // evaluated whether there is one or not, with tau = 0 if not: without
@@ -322,7 +324,7 @@ __device__ __forceinline__ void flux_compact(float a0, float a1, int dc0, int dc
                                              Sink &&sink) {
   using SH = Flux32Shape<ORDER>;
   constexpr int S = SH::S, BX = S + 1;
-  const int IA = exact_base<ORDER>(a0), JA = exact_base<ORDER>(a1), IB = dc0 + exact_base<ORDER>(b0);
+  const int IA = base_index<ORDER>(a0), JA = base_index<ORDER>(a1), IB = dc0 + base_index<ORDER>(b0);
   const bool wide = IB != IA;
   open_box<COMP == 0 ? BX - 1 : BX, COMP == 0 ? S : S - 1>(sink, IA + SH::OFF, JA + SH::OFF, 0);
   const double tK = d_add(K, kRound);
@@ -411,9 +413,7 @@ __device__ __forceinline__ void flux_compact(float a0, float a1, int dc0, int dc
 // (dc0, dc1) = new cell - old cell, (b0, b1): end offset in the new cell;
 // K = q * scale, Kint = its integer value.  COMP selects the emitted
 // component; sink(i, j, v) gets old-cell-relative Jx / Jy indices.
-// FAST (the compact form): the caller has checked that the move keeps its y base
-// index and advances its x base index by 0 or 1; it then runs unless |K| is
-// too large for it.
+// FAST: moves that allow the compact form take it.
 // Returns false when the move spans more than one base index on an axis
 // (more than one cell for CFL <= 1); nothing is emitted then.
 template <int ORDER, int COMP, bool FAST, class Sink>
@@ -421,7 +421,7 @@ __device__ __forceinline__ bool flux_particle(float a0, float a1, int dc0, int d
                                               long long Kint, Sink &&sink) {
   using SH = Flux32Shape<ORDER>;
   if constexpr (FAST) {
-    if (!(fabs(K) < kRoundMax))
+    if (!compact_form<ORDER>(a0, a1, dc0, dc1, b0, b1, K))
       return flux_particle<ORDER, COMP, false>(a0, a1, dc0, dc1, b0, b1, K, Kint, sink);
     flux_compact<ORDER, COMP>(a0, a1, dc0, dc1, b0, b1, K, sink);
     return true;

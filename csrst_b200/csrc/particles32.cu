@@ -258,12 +258,10 @@ __device__ __forceinline__ void push32_range(const Push32Args &a, const Work &wo
       }
       const int wi = m.ci - WP0, wj = m.cj - WP1;
       tile.template rebase<false>(m.ok, wi, wj, a.acc, L0, L1);
-      // the compact form when every particle of the warp keeps its y base index
-      // and advances by at most one x base index
-      const int dx = m.ni - m.ci + base_index<ORDER>(m.o0) - base_index<ORDER>(m.a0);
+      // the compact form when every particle of the warp allows it
       const double K = (double)m.q * a.acc_scale;
-      const bool fast = !m.ok || ((unsigned)dx <= 1u && fabs(K) < kRoundMax &&
-                                  m.nj - m.cj + base_index<ORDER>(m.o1) == base_index<ORDER>(m.a1));
+      const bool fast =
+          !m.ok || compact_form<ORDER>(m.a0, m.a1, m.ni - m.ci, m.nj - m.cj, m.o0, m.o1, K);
       const bool all_fast = __all_sync(0xffffffffu, fast);
       if (m.ok) {
         TileSink<Tile> sink(tile, wi, wj, a.acc, L0, L1);
