@@ -777,6 +777,15 @@ cudaError_t alloc_old32(csrst_handle *h) {
   return e;
 }
 
+// Scratch of the fused sweep's fix-up: the window's footprint widened by two
+// cells and the cells its sub-steps read (launch_yee_fused).  The fused step
+// runs where it is there (fused_ok).
+cudaError_t alloc_zfix(csrst_handle *h) {
+  h->zpitch = h->L0 + 6;
+  h->zrows = h->L1 + 7;
+  return cudaMalloc(&h->zfix, 4 * (size_t)h->zpitch * h->zrows * (h->fp32 ? sizeof(float) : sizeof(double)));
+}
+
 int need_bunch(csrst_handle *h) {
   if (!h) return CSRST_E_ARG;
   if (h->n <= 0 || !(h->win || h->winf)) return fail(h, CSRST_E_NO_PARTICLES, "no bunch loaded");
@@ -1081,11 +1090,7 @@ int csrst_load_particles(csrst_handle *h, const double *x, const double *y, cons
   }
   CK(cudaMalloc(&h->acc, 2 * (size_t)h->L0 * h->L1 * sizeof(unsigned long long)));
   CK(cudaMemsetAsync(h->acc, 0, 2 * (size_t)h->L0 * h->L1 * sizeof(unsigned long long), h->s));
-  // scratch of the fused sweep's fix-up: the window's footprint widened by
-  // two cells and the cells its sub-steps read (launch_yee_fused)
-  h->zpitch = h->L0 + 6;
-  h->zrows = h->L1 + 7;
-  CK(cudaMalloc(&h->zfix, 4 * (size_t)h->zpitch * h->zrows * (h->fp32 ? sizeof(float) : sizeof(double))));
+  CK(alloc_zfix(h));
   // PartBunch::sortParticles: y slice of the window, then x (stable radix sorts)
   {
     unsigned long long *kx = nullptr, *kx2 = nullptr;
@@ -2505,6 +2510,7 @@ int csrst_checkpoint_read(csrst_handle *h, const char *path, long long *step, do
     CK(cudaMalloc(&h->scratch, 6 * wp * es));
   }
   CK(cudaMalloc(&h->acc, 2 * (size_t)h->L0 * h->L1 * sizeof(unsigned long long)));
+  CK(alloc_zfix(h));
   P = ck_plan(h);
   for (auto &pl : P.window)
     if (!ck_get_dev(f, pl.first, pl.second, buf, h->s)) return bad(CSRST_E_IO, "truncated file (window)");
