@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "../../include/csrst.h"
 #include "nn.h"
 
@@ -146,9 +148,55 @@ struct Seq {
   }
 };
 
-bool valid(const csrst_fno *f, const int *err) {
-  return f && err && f->width > 0 && f->modes > 0 && f->layers > 0 && f->nout > 0 && f->batch > 0 && f->w && f->w16 &&
-         (long long)f->batch * kBins <= 0x7fffffffll;
+// A call is refused before its first launch when a size is one that a kernel of
+// the sequence does not take, or a buffer it reads or writes is missing or, where
+// its kernels read it 16 bytes at a time or as a product's operand, not 16-byte aligned.
+bool there(std::initializer_list<const void *> ps) {
+  for (const void *p : ps)
+    if (!p) return false;
+  return true;
+}
+bool aligned(std::initializer_list<const void *> ps) {
+  for (const void *p : ps)
+    if (!p || ((uintptr_t)p & 15)) return false;
+  return true;
+}
+bool aligned(const void *const *table, int n) {
+  if (!table) return n <= 0;
+  for (int k = 0; k < n; ++k)
+    if (!aligned({table[k]})) return false;
+  return true;
+}
+
+// The network itself (any sequence).
+bool valid(const csrst_fno *f) {
+  constexpr long long most = 0x7fffffffll;
+  if (!f || f->width <= 0 || f->width % 64 || f->modes <= 0 || f->modes % 32 || f->layers < 1 || f->nout < 16 ||
+      f->nout > 64 || f->nout % 16 || f->batch <= 0)
+    return false;
+  // (rows, columns and output counts go to the kernels as ints; the modes are a batch)
+  return (long long)f->batch * kBins <= most && (long long)f->batch * f->width <= most &&
+         (long long)f->width * f->width <= most && f->modes <= 65535 && f->w && aligned({f->w16});
+}
+
+bool can_forward(const csrst_fno *f) {
+  if (!valid(f)) return false;
+  const int L = f->layers;
+  if (!aligned({f->F16, f->G16, f->U16, f->Zp16, f->A1_16}) || !f->Z16 || !aligned(f->Mk16, L) || !f->Mk16 || !f->V16 ||
+      !aligned(f->V16, f->train ? L + 1 : 2))
+    return false;
+  if (!f->train) return true;
+  // weight gradients are products over batch columns; R rows go to the transposes 32 to a block
+  return f->batch % 64 == 0 && f->batch * (kBins / 32) <= 65535 && aligned({f->A1pre, f->A1t16}) && f->Vg16 && f->Ut16 &&
+         aligned(f->Vg16, L + 1) && aligned(f->Ut16, L) && aligned((const void *const *)f->Hfull, L - 1);
+}
+
+bool can_backward(const csrst_fno *f) {
+  return can_forward(f) && f->train && f->g && f->WT16 && f->MkT16 && aligned(f->WT16, f->layers) &&
+         aligned(f->MkT16, f->layers) &&
+         aligned({f->Q1T16, f->Q2T16, f->FT16, f->GT16, f->Xt16, f->dOut, f->dOut16, f->dOutT16, f->dA1, f->dH, f->dH16,
+                  f->dHt16, f->dV, f->dVn, f->dZ16, f->dZt16, f->dS16}) &&
+         there({f->out, f->dSk16, f->dMk, f->part, f->cpart, f->lpart, f->loss});
 }
 
 void forward(Seq &q, const void *X16, float *out) {
@@ -281,14 +329,14 @@ void backward(Seq &q, const void *X16, const float *T, const float *Wt) {
 extern "C" {
 
 int csrst_fno_forward(const csrst_fno *f, const void *X16, float *out, int *err, void *stream) {
-  if (!valid(f, err) || !X16 || !out) return CSRST_E_ARG;
+  if (!can_forward(f) || !err || !aligned({X16}) || !out) return CSRST_E_ARG;
   Seq q(*f, err, stream, f->train);
   if (q.ok()) forward(q, X16, out);
   return q.rc;
 }
 
 int csrst_fno_backward(const csrst_fno *f, const void *X16, const float *T, const float *Wt, int *err, void *stream) {
-  if (!valid(f, err) || !f->train || !f->g || !X16 || !T) return CSRST_E_ARG;
+  if (!can_backward(f) || !err || !aligned({X16}) || !T) return CSRST_E_ARG;
   Seq q(*f, err, stream, true);
   if (q.ok()) backward(q, X16, T, Wt);
   return q.rc;
@@ -296,9 +344,12 @@ int csrst_fno_backward(const csrst_fno *f, const void *X16, const float *T, cons
 
 int csrst_fno_refresh(const csrst_fno *f, long long n, void *stream) {
   int none = 0;
-  if (!valid(f, &none) || n <= 0) return CSRST_E_ARG;
+  if (!valid(f) || !there({f->WT16, f->Mk16, f->MkT16, f->Q1T16, f->Q2T16}) || !aligned(f->WT16, f->layers) ||
+      !aligned(f->Mk16, f->layers) || !aligned(f->MkT16, f->layers))
+    return CSRST_E_ARG;
   Seq q(*f, &none, stream, false);
   const long long w = q.w;
+  if (n < q.oq2() + f->nout) return CSRST_E_ARG;  // w16 is read up to there
   q.cast(f->w, f->w16, n);
   for (int l = 0; l < f->layers; ++l) {
     q.transpose16(q.p16(q.oW(l)), f->WT16[l], 1, w, w, w);

@@ -307,8 +307,14 @@ int csrst_nn_spectral_unpack(const float *dmk, int modes, int ch, float *dwr, fl
  * of the products and kernels above: the device pointers of one network and of the buffers of one
  * batch size, read during the call only.  w, g, w16: the flat parameters (FP32), their gradient and
  * BF16 copy in the order P [width][64], p, per layer W [width][width], b, Wr and Wi
- * [modes][width][width], then Q1, q1, Q2 [nout][width], q2.  Fields from Vg16 on are read with train != 0 alone.
- * R = 256 batch rows. */
+ * [modes][width][width], then Q1, q1, Q2 [nout][width], q2 (in w and g padded to 64 values).  Fields from
+ * Vg16 on are read with train != 0 alone.  R = 256 batch rows.
+ *
+ * Limits: width a multiple of 64, modes of 32 (at most 65535), nout of 16 in 16 .. 64, R, batch width and
+ * width^2 below 2^31; with train batch a multiple of 64, at most 8128.  Every array that a call reads or
+ * writes is there; X16, w16, the BF16 arrays but Z16 and dSk16, and the FP32 ones that the backward pass takes through
+ * an activation (Hfull, A1pre, dOut, dA1, dH, dV, dVn) are 16-byte aligned.  Anything else is CSRST_E_ARG, with
+ * nothing launched. */
 typedef struct {
   int width, modes, layers, nout, batch, train;
   const float *w;
