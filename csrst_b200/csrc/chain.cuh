@@ -28,7 +28,9 @@ bool launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStr
   c.stream = s;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, k, std::forward<A>(args)...) == cudaSuccess;
+  if (cudaLaunchKernelEx(&c, k, std::forward<A>(args)...) == cudaSuccess) return true;
+  cudaGetLastError();  // reported by this call: it is not the next one's
+  return false;
 }
 
 }  // namespace csrst
