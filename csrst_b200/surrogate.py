@@ -146,15 +146,18 @@ class _Buffers:
         self.cpart = torch.empty(max(B * max(w, 64), ((R // KSPLIT + 255) // 256) * w * max(w, NFEAT)), **f32)
         self.lpart = torch.empty(256, dtype=torch.float64, device=dev)
         self.loss = torch.zeros(1, dtype=torch.float64, device=dev)
-        self.side = torch.cuda.Stream(dev)  # joined to the caller's stream within each call
+
+    # the training step's second stream, joined to the caller's within each call; made by
+    # the first step, so that a network can be unpickled where there is no GPU
+    side = None
+
+    def side_stream(self):
+        if self.side is None:
+            self.side = torch.cuda.Stream(self.loss.device)
+        return self.side.cuda_stream
 
     def __getstate__(self):   # a copy gets a side stream of its own
         return {k: v for k, v in vars(self).items() if k != "side"}
-
-    def __setstate__(self, d):
-        vars(self).update(d)
-        if self.train:
-            self.side = torch.cuda.Stream(self.loss.device)
 
 
 class FNO:
@@ -236,10 +239,10 @@ class FNO:
                     v = _ptrs(v)
                     n.keep.append(v)
                     setattr(n, k, C.addressof(v))
-                elif k == "side":
-                    n.side = v.cuda_stream
-                elif k != "train":
+                elif torch.is_tensor(v):
                     setattr(n, k, v.data_ptr())
+            if bf.train:
+                n.side = bf.side_stream()
         return n
 
     def _buf(self, B, train):
