@@ -1645,31 +1645,41 @@ void launch_reset_outside(FieldArgsT<T> a, const int *cutidx, cudaStream_t s) {
 
 // --- fused sweep: host side ---------------------------------------------------
 
-EncodeTiled tensor_map_encoder() {
-  static const EncodeTiled fn = [] {
+bool encode_tiled(CUtensorMap *m, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims,
+                  const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle) {
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode fn = [] {
     void *p = nullptr;
     cudaDriverEntryPointQueryResult q{};
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
         q != cudaDriverEntryPointSuccess)
-      return (EncodeTiled) nullptr;
-    return reinterpret_cast<EncodeTiled>(p);
+      return (Encode) nullptr;
+    return reinterpret_cast<Encode>(p);
   }();
-  return fn;
+  if (!fn) return false;
+  static const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
+  auto encode = [&] {
+    return fn(m, type, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, ones,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  if (encode()) return true;
+  // a thread that has made no runtime call yet has no context of its device
+  // current, which the driver's call wants and the runtime's calls see to
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && encode();
 }
 
 // Row-major 2-D map of w x h elements, rows pitch_bytes apart, box bw x bh;
 // reads outside the tensor return zero.
 static bool encode_2d(CUtensorMap *m, CUtensorMapDataType dt, const void *base, uint64_t w, uint64_t h,
                       uint64_t pitch_bytes, uint32_t bw, uint32_t bh) {
-  const EncodeTiled enc = tensor_map_encoder();
-  if (!enc) return false;
   const cuuint64_t dims[2] = {w, h};
   const cuuint64_t strides[1] = {pitch_bytes};
   const cuuint32_t box[2] = {bw, bh};
-  const cuuint32_t es[2] = {1, 1};
-  return enc(m, dt, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode_tiled(m, dt, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 // The tile arguments of one sweep (tensor maps over a's static planes, the

@@ -843,16 +843,12 @@ long long g_wait_polls = kSpin;
 // apart): rows x K (x batch), box 64 x 64.
 bool encode_operand(CUtensorMap *m, int *rank3, const __nv_bfloat16 *p, int K, long long rows, long long ld,
                     long long stride, int batch, int box_rows, bool mn = false) {
-  const EncodeTiled enc = tensor_map_encoder();
-  if (!enc) return false;
   *rank3 = batch > 1 && stride != 0;
   const cuuint64_t dims[3] = {(cuuint64_t)(mn ? rows : K), (cuuint64_t)(mn ? K : rows), (cuuint64_t)batch};
   const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)stride * 2};
   const cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)(mn ? 64 : box_rows), 1};
-  const cuuint32_t es[3] = {1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, *rank3 ? 3 : 2, const_cast<__nv_bfloat16 *>(p), dims, strides,
-             box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, *rank3 ? 3 : 2, p, dims, strides, box,
+                      CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int BN, int FORM>

@@ -7,12 +7,11 @@
 
 namespace csrst {
 
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled of the driver, found once through the runtime (host).
-EncodeTiled tensor_map_encoder();
+// Tiled tensor map of `rank` dimensions (fields.cu): cuTensorMapEncodeTiled of
+// the driver, found once through the runtime, with unit element strides, 256-byte L2
+// promotion and zero fill.  Any thread may call it.
+bool encode_tiled(CUtensorMap *m, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims,
+                  const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle);
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
