@@ -28,6 +28,7 @@ fixed order, so a training run repeats bit for bit.
 """
 import ctypes as C
 import math
+import threading
 
 import numpy as np
 import torch
@@ -119,6 +120,7 @@ class _Buffers:
         self.A1_16 = torch.empty(R, w, **bf)
         self.out = torch.empty(R, net.nout, **f32)
         self.train = train
+        self.lock = threading.Lock()  # held while a pass's launches go out
         if not train:
             return
         self.Vg16 = [torch.empty(w, R, **bf) for _ in range(L + 1)]
@@ -156,8 +158,11 @@ class _Buffers:
             self.side = torch.cuda.Stream(self.loss.device)
         return self.side.cuda_stream
 
-    def __getstate__(self):   # a copy gets a side stream of its own
-        return {k: v for k, v in vars(self).items() if k != "side"}
+    def __getstate__(self):   # a copy gets a side stream and a lock of its own
+        return {k: v for k, v in vars(self).items() if k not in ("side", "lock")}
+
+    def __setstate__(self, d):
+        vars(self).update(d, lock=threading.Lock())
 
 
 class FNO:
@@ -246,9 +251,12 @@ class FNO:
         return n
 
     def _buf(self, B, train):
-        key = (B, train)
+        """The buffers of a batch of B members.  Inference has a set per stream: passes on two
+        streams run beside each other (a training pass writes the network's gradient, so two
+        of them are not for running at a time anyway)."""
+        key = (B, True) if train else (B, False, _stream().value)
         if key not in self._bufs:
-            self._bufs[key] = _Buffers(self, B, train)
+            self._bufs.setdefault(key, _Buffers(self, B, train))
         return self._bufs[key]
 
     # ---- forward ----
@@ -263,7 +271,8 @@ class FNO:
         for a in range(0, N, chunk):
             B = min(chunk, N - a)
             bf = self._buf(B, False)
-            self._forward(self._net(bf, B), X[a:a + B].reshape(B * NBINS, NFEAT), out[a:a + B])
+            with bf.lock:  # threads on one stream: one pass's launches after another's
+                self._forward(self._net(bf, B), X[a:a + B].reshape(B * NBINS, NFEAT), out[a:a + B])
         return out
 
     # ---- backward ----
