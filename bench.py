@@ -204,8 +204,8 @@ def time_mode(args, cfg, bunch, world, fp32, clocks):
     ms = max_over_ranks(t0.elapsed_time(t1), world)
     if world > 1:
         torch.distributed.barrier()
-    # ---- kernel attribution: the same steps' kernels, eagerly, with CUDA
-    # events between the groups on the library's stream (csrst_step_timed) ----
+    # ---- kernel attribution: eager steps with CUDA events between the groups,
+    # one group after another (csrst_step_timed; the timed steps overlap them) ----
     groups = {"push": 0.0, "yee": 0.0, "move": 0.0}
     ksteps = min(args.steps, 10)
     for _ in range(ksteps):

@@ -701,10 +701,9 @@ bool step_tail_async(csrst_handle *h) {
   return true;
 }
 
-void mark_on(csrst_handle *h, int k, cudaStream_t s) {
-  if (h->tev) cudaEventRecord(h->tev[k], s);
+void mark(csrst_handle *h, int k) {
+  if (h->tev) cudaEventRecord(h->tev[k], h->s);
 }
-void mark(csrst_handle *h, int k) { mark_on(h, k, h->s); }
 
 // TETMSolver::updateField_firstStep + updateField_secondStep + moveMesh.
 // Events 0..7 (csrst_step_timed) bracket the pushes, the field work of each
@@ -722,20 +721,23 @@ int step_async(csrst_handle *h) {
       h->prepped = false;
       return rc;
     }
+    // the second push reads the window, which the fix-up alone writes: it
+    // follows the fix-up on s2 while the tiles run on.  A timed step runs its
+    // groups one after another on s, the window move as a launch of its own
+    const bool timed = h->tev != nullptr;
+    auto join = [&]() {
+      cudaEventRecord(h->join, h->s2);
+      cudaStreamWaitEvent(h->s, h->join, 0);
+    };
+    if (timed) join();
     mark(h, 2);
     drift_back(h);
-    // the second push reads the window, which the fix-up alone writes: it
-    // follows the fix-up on s2 while the tiles run on
-    mark_on(h, 3, h->s2);
-    push_async(h, 1, h->s2);
-    mark_on(h, 4, h->s2);
-    cudaEventRecord(h->join, h->s2);
-    cudaStreamWaitEvent(h->s, h->join, 0);
-    if (step_tail_async(h)) {
-      mark(h, 5);
-      mark(h, 6);
-      mark(h, 7);
-      return CSRST_OK;
+    mark(h, 3);
+    push_async(h, 1, timed ? h->s : h->s2);
+    mark(h, 4);
+    if (!timed) {
+      join();
+      if (step_tail_async(h)) return CSRST_OK;
     }
     window_ey_async(h);
   } else {

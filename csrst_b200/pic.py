@@ -191,8 +191,8 @@ class Simulation:
         self._ck(lib().csrst_step(self.h, n))
 
     def step_timed(self):
-        """One step with device times of its kernel groups (ms): push,
-        fields, move, total."""
+        """One step with device times of its kernel groups (ms), which run one
+        after another here: push, fields, move, total."""
         out = np.zeros(4)
         self._ck(lib().csrst_step_timed(self.h, ptr(out)))
         return dict(zip(("push", "fields", "move", "total"), out.tolist()))

@@ -166,13 +166,13 @@ int csrst_step_second(csrst_handle *h);
  * another (the sets swap every step; every read and write of the fields goes
  * to the current set), bit for bit what the sub-step calls above give. */
 int csrst_step(csrst_handle *h, int nsteps);
-/* One step as csrst_step takes it (same kernels, launched eagerly) with CUDA
- * events between its kernel groups; waits for it and returns the device
- * times in ms4 [ms]: both pushes, the field work (the fused sweep, or the
+/* One step, bit for bit what csrst_step gives, launched eagerly with CUDA events
+ * between its kernel groups, one group after another; waits for it and returns the
+ * device times in ms4 [ms]: both pushes, the field work (the fused sweep, or the
  * four sub-steps with their exchanges, and the window's Ey), the window move,
- * and the whole step.  In the fused step the second push runs beside the
- * sweep's tiles, so the groups overlap and their sum is above the whole; where the
- * window's Ey and its move are one launch, it counts as field work and the move is 0. */
+ * and the whole step.  In csrst_step the second push runs beside the sweep's tiles,
+ * and the window's Ey, its move and the next push's set-up are one launch where the
+ * window is not too large, so a step there takes less than the groups' sum here. */
 int csrst_step_timed(csrst_handle *h, double *ms4);
 /* Polls a fused-sweep tile makes in its staging wait (the TMA copies of its
  * fields) before it gives up, writes nothing and reports CSRST_E_STAGING at
