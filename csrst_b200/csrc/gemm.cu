@@ -866,6 +866,8 @@ int start_gemm(const GemmArgs &a, int dev, int grid, cudaStream_t s) {
 template <int BN>
 int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csrst_gemm_epilogue &ep, int *err,
                 cudaStream_t s) {
+  const long long tiles = tile_count(M, N, batch, kBM, BN);
+  if (tiles < 0) return CSRST_E_ARG;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
                                                 cudaSuccess)
@@ -878,10 +880,9 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   a.nk2 = g1.nk;
   a.M = M;
   a.N = N;
-  a.tilesM = (M + kBM - 1) / kBM;
-  a.tilesN = (N + BN - 1) / BN;
-  if ((long long)batch * a.tilesM > 0x7fffffffll / a.tilesN) return CSRST_E_ARG;  // 2^31 tiles hold 2^43 outputs
-  a.ntiles = batch * a.tilesM * a.tilesN;
+  a.tilesM = (int)(((long long)M + kBM - 1) / kBM);
+  a.tilesN = (int)(((long long)N + BN - 1) / BN);
+  a.ntiles = (int)tiles;
   a.dN = make_div(a.tilesN);
   a.dM = make_div(a.tilesM);
   a.md = make_div(ep.md);
@@ -906,7 +907,7 @@ int launch_gemm(const Seg &g0, const Seg &g1, int M, int N, int batch, const csr
   }
   a.bias4 = ep.bias && !(reinterpret_cast<uintptr_t>(ep.bias) & 15);
   const int grid = a.ntiles < sms ? a.ntiles : sms;
-switch (form_of(a)) {
+  switch (form_of(a)) {
     case kRuns: return start_gemm<BN, kRuns>(a, dev, grid, s);
     case kAddRuns: return start_gemm<BN, kAddRuns>(a, dev, grid, s);
     default: return start_gemm<BN, kAnyForm>(a, dev, grid, s);

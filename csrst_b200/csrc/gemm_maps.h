@@ -128,4 +128,13 @@ inline RunShape run_shape(const long long *rdel, const long long *cdel, int L) {
   return RunShape{-1, 0};
 }
 
+// Output tiles of bm x bn of a launch, or -1 where they are more than the
+// kernel's 32-bit tile index takes: it steps by the grid, so the last step may go
+// past the last tile by as much (2^31 tiles hold 2^43 outputs).
+inline long long tile_count(int M, int N, int batch, int bm, int bn) {
+  constexpr long long kMost = 0x7fffffffll - 0xffff;
+  const long long m = ((long long)M + bm - 1) / bm, n = ((long long)N + bn - 1) / bn;
+  return (long long)batch * m > kMost / n ? -1 : batch * m * n;
+}
+
 }  // namespace csrst
