@@ -51,9 +51,13 @@
 namespace csrst {
 namespace {
 
+// The stencil is symmetric (E of a column is W of the next, N of a row S of the
+// next) and 0 towards inactive cells.  D and S of a coarse level are gone once
+// its factors and the next level are there.
 struct Level {
   int nx, ny;
-  double *D, *W, *E, *S, *N;  // stencil; off-diagonals are 0 towards inactive cells
+  double *D, *W, *S;
+  double d0;                  // the finest level's D on its active rows (D is nullptr there, 1 on the others)
   uint8_t *act;
   double *u, *f;              // correction, right-hand side
   double *fac;                // line factors (LineFactors)
@@ -78,19 +82,16 @@ __global__ void k_classes(const uint8_t *mask, const int *cutidx, const CutCellD
   act[k] = g && i < maxX;
 }
 
-__global__ void k_coeff0(Level L, double EW, double NS, double Dc) {
+__global__ void k_coeff0(Level L, double EW, double NS) {
   const long long k = gtid();
   if (k >= (long long)L.nx * L.ny) return;
   const int i = (int)(k / L.ny), j = (int)(k % L.ny);
   if (!L.act[k]) {
-    L.D[k] = 1.0; L.W[k] = L.E[k] = L.S[k] = L.N[k] = 0.0;
+    L.W[k] = L.S[k] = 0.0;
     return;
   }
-  L.D[k] = Dc;
   L.W[k] = (i > 0 && L.act[k - L.ny]) ? EW : 0.0;
-  L.E[k] = (i + 1 < L.nx && L.act[k + L.ny]) ? EW : 0.0;
   L.S[k] = (j > 0 && L.act[k - 1]) ? NS : 0.0;
-  L.N[k] = (j + 1 < L.ny && L.act[k + 1]) ? NS : 0.0;
 }
 
 // Galerkin coarse stencil of a pair of columns (2I, 2I+1).
@@ -102,23 +103,25 @@ __global__ void k_coarsen(Level F, Level C) {
   const bool ha = F.act[a], hb = 2 * I + 1 < F.nx && F.act[b];
   if (!ha && !hb) {
     C.act[k] = 0;
-    C.D[k] = 1.0; C.W[k] = C.E[k] = C.S[k] = C.N[k] = 0.0;
+    C.D[k] = 1.0; C.W[k] = C.S[k] = 0.0;
     return;
   }
-  double D = 0.0, W = 0.0, E = 0.0, S = 0.0, N = 0.0;
-  if (ha) { D += F.D[a] + F.E[a]; W += F.W[a]; S += F.S[a]; N += F.N[a]; }
-  if (hb) { D += F.D[b] + F.W[b]; E += F.E[b]; S += F.S[b]; N += F.N[b]; }
+  double D = 0.0, W = 0.0, S = 0.0;
+  const double E = 2 * I + 1 < F.nx ? F.W[b] : 0.0;  // between the two
+  if (ha) { D += (F.D ? F.D[a] : F.d0) + E; W += F.W[a]; S += F.S[a]; }
+  if (hb) { D += (F.D ? F.D[b] : F.d0) + E; S += F.S[b]; }
   C.act[k] = 1;
-  C.D[k] = 0.5 * D; C.W[k] = 0.5 * W; C.E[k] = 0.5 * E; C.S[k] = 0.5 * S; C.N[k] = 0.5 * N;
+  C.D[k] = 0.5 * D; C.W[k] = 0.5 * W; C.S[k] = 0.5 * S;
 }
 
+// A u at an active row of the finest level.
 __device__ __forceinline__ double apply_at(const Level &L, const double *u, long long k) {
   const int i = (int)(k / L.ny), j = (int)(k % L.ny);
-  double v = L.D[k] * u[k];
+  double v = L.d0 * u[k];
   if (i > 0) v += L.W[k] * u[k - L.ny];
-  if (i + 1 < L.nx) v += L.E[k] * u[k + L.ny];
+  if (i + 1 < L.nx) v += L.W[k + L.ny] * u[k + L.ny];
   if (j > 0) v += L.S[k] * u[k - 1];
-  if (j + 1 < L.ny) v += L.N[k] * u[k + 1];
+  if (j + 1 < L.ny) v += L.S[k + 1] * u[k + 1];
   return v;
 }
 
@@ -152,7 +155,9 @@ __global__ void __launch_bounds__(128) k_factor(Level L) {
   double *F = L.fac + (size_t)col * line_factors(ny) + lane;
   auto row = [&](int j, double &a, double &b, double &c) {
     const bool in = j < ny;
-    a = in ? L.S[base + j] : 0.0; b = in ? L.D[base + j] : 1.0; c = in ? L.N[base + j] : 0.0;
+    a = in ? L.S[base + j] : 0.0;
+    b = !in ? 1.0 : L.D ? L.D[base + j] : L.act[base + j] ? L.d0 : 1.0;
+    c = j + 1 < ny ? L.S[base + j + 1] : 0.0;
   };
   auto at = [&](int q, int k) -> double & { return F[(size_t)(k * kRowFactors + q) * 32]; };
   // interior rows k = 0 .. m - 2: pivots, v's forward sweep
@@ -240,12 +245,12 @@ __device__ __forceinline__ void line_column(const Level &L, const Level *fine, c
       if (!in) continue;
       if (restricted) {  // (fw, ew) and (fe, ee): the finer level's even column
         if (fwest) { fw[t] = __ldg(fine->W + fb + j); ew[t] = fine->u[fb + j - ny]; }
-        if (feast) { fe[t] = __ldg(fine->E + fb + j); ee[t] = fine->u[fb + j + ny]; }
+        if (feast) { fe[t] = __ldg(fine->W + fb + j + ny); ee[t] = fine->u[fb + j + ny]; }
       } else {
         d[t] = L.f[k];
       }
       if (west) { cw[t] = __ldg(L.W + k); uw[t] = L.u[k - ny]; }
-      if (east) { ce[t] = __ldg(L.E + k); ue[t] = L.u[k + ny]; }
+      if (east) { ce[t] = __ldg(L.W + k + ny); ue[t] = L.u[k + ny]; }
       if (MODE == kUp1) {
         if (west) ew[t] = coarse->u[(size_t)((col - 1) / 2) * ny + j];
         if (east) ee[t] = coarse->u[(size_t)((col + 1) / 2) * ny + j];
@@ -656,20 +661,28 @@ struct Work {
   unsigned *done;
   std::vector<Level> lv;
   uint8_t *good;
-  double *b, *f, *x, *r, *d, *q, *phi[3];
-  unsigned long long *acc;
+  double *b, *r, *d, *q, *phi[3];
+  double *f;                // the right-hand side, until the first search direction takes its place (d)
+  unsigned long long *acc;  // the charge, until the first A d does (q)
   void carve(Arena &A, int Nx, int Ny) {
     const size_t m = (size_t)Nx * Ny;
     part = A.get<double>(std::max(kDotBlocks, 3 * kPsumBlocks)); scal = A.get<double>(8); done = A.get<unsigned>(1);
     good = A.get<uint8_t>(m);
-    for (double **p : {&b, &f, &x, &r, &d, &q, &phi[0], &phi[1], &phi[2]}) *p = A.get<double>(m);
-    acc = A.get<unsigned long long>(m);
+    for (double **p : {&b, &r, &d, &q, &phi[0], &phi[1], &phi[2]}) *p = A.get<double>(m);
+    f = d;
+    static_assert(sizeof(unsigned long long) == sizeof(double), "acc shares q's place");
+    acc = reinterpret_cast<unsigned long long *>(q);
     lv.clear();
+    // D and S of the coarse levels, in turns: a level's are read by its factors and the next level only
+    const size_t c1 = (size_t)((Nx + 1) / 2) * Ny, c2 = (size_t)((Nx + 3) / 4) * Ny;
+    double *D[2] = {A.get<double>(c1), A.get<double>(c2)}, *S[2] = {A.get<double>(c1), A.get<double>(c2)};
     for (int nx = Nx;; nx = (nx + 1) / 2) {
       Level L{};
       L.nx = nx; L.ny = Ny;
       const size_t c = (size_t)nx * Ny;
-      for (double **p : {&L.D, &L.W, &L.E, &L.S, &L.N, &L.u}) *p = A.get<double>(c);
+      for (double **p : {&L.W, &L.u}) *p = A.get<double>(c);
+      if (lv.empty()) L.S = A.get<double>(c);
+      else { L.D = D[(lv.size() - 1) & 1]; L.S = S[(lv.size() - 1) & 1]; }
       L.act = A.get<uint8_t>(c);
       L.f = lv.empty() ? r : A.get<double>(c);  // the finest level's right-hand side is CG's residual
       L.fac = A.get<double>((size_t)nx * line_factors(Ny));
@@ -773,10 +786,12 @@ int poisson_initial_fields(const PoissonInput &in, PoissonReport *rep, cudaStrea
   const long long maxX = (long long)(size_t)(in.b.Lb / in.b.hr0);
 
   k_classes<<<blocks_for(m), 256, 0, s>>>(in.mask, in.cutidx, in.cells, Nx, Ny, maxX, w.good, lv[0].act);
-  k_coeff0<<<blocks_for(m), 256, 0, s>>>(lv[0], EW, NS, Dc);
-  for (size_t l = 1; l < lv.size(); ++l)
-    k_coarsen<<<blocks_for((long long)lv[l].nx * Ny), 256, 0, s>>>(lv[l - 1], lv[l]);
-  for (const Level &L : lv) k_factor<<<(L.nx + 3) / 4, 128, 0, s>>>(L);
+  w.lv[0].d0 = Dc;
+  k_coeff0<<<blocks_for(m), 256, 0, s>>>(lv[0], EW, NS);
+  for (size_t l = 0; l < lv.size(); ++l) {
+    if (l > 0) k_coarsen<<<blocks_for((long long)lv[l].nx * Ny), 256, 0, s>>>(lv[l - 1], lv[l]);
+    k_factor<<<(lv[l].nx + 3) / 4, 128, 0, s>>>(lv[l]);
+  }
   Solver sv(lv, s);
   if ((e = sv.opt_in()) != cudaSuccess) return fail("line solver shared memory", e);
   const Scalars S{part, scal, w.done};
@@ -790,8 +805,9 @@ int poisson_initial_fields(const PoissonInput &in, PoissonReport *rep, cudaStrea
   const double full = (in.dt / 2) * kC, back = (-in.dt / 2) * kC, mv = -0.5 * hr0 / gamma;
   const unsigned pg = blocks_for(in.n) < 4096 ? blocks_for(in.n) : 4096;
   const double tols[3] = {in.tol_first, in.tol_rest, in.tol_rest};
-  double *x = w.x, *r = w.r, *z = lv[0].u;
+  double *r = w.r, *z = lv[0].u;
   for (int sol = 0; sol < 3; ++sol) {
+    double *x = w.phi[sol];
     // right-hand side of this solve
     cudaMemsetAsync(w.acc, 0, m * sizeof(unsigned long long), s);
     const int mode = sol;  // 0: R + dt/2 drift, 1: shifted by -hx/2, 2: R

@@ -111,7 +111,9 @@ int csrst_load_particles(csrst_handle *h, const double *x, const double *y, cons
  * GPU replaces Trilinos ML + BlockCG.  tol_first / tol_rest: relative residual
  * of the first solve (main.cpp:94, 1e-12) and of the other two (1e-6);
  * max_iter per solve (main.cpp:93, 500).  report8 (may be NULL): gamma,
- * iterations and relative residual of each solve, multigrid levels. */
+ * iterations and relative residual of each solve, multigrid levels.  Device
+ * memory during the call: some 210 to 220 bytes a mesh cell for 500 rows and more,
+ * up to 290 for 100, in one allocation (csrst_release_memory). */
 int csrst_initial_fields(csrst_handle *h, double tol_first, double tol_rest, int max_iter, double *report8);
 /* Current bunch in the handle's (cell-sorted) order. */
 int csrst_get_particles(csrst_handle *h, double *x, double *y, double *px, double *py);
@@ -185,8 +187,11 @@ int csrst_set_staging_wait_limit(long long polls);
 /* A handle's bunch arrays and the temporaries of csrst_load_particles come
  * from a stream-ordered memory pool the library keeps per device: memory a
  * destroyed handle or a reload frees stays in the pool for the next load
- * (no device-wide waits for cudaMalloc / cudaFree).  This returns the
- * pool's unused memory of the current device to the driver. */
+ * (no device-wide waits for cudaMalloc / cudaFree).  So do the scratch of
+ * csrst_initial_fields and FP32 mode's staging of field reads and writes, up to
+ * 1 GiB each; larger ones go back to the driver at the call's end.  The driver
+ * takes unused pool memory for other allocations of the process by itself; for
+ * other processes this returns the pool's unused memory of the current device. */
 int csrst_release_memory(void);
 
 /* Batched ensemble (no reference counterpart: the reference runs one bunch
