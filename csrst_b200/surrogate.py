@@ -93,7 +93,8 @@ def _ptrs(ts):
 
 
 class _Buffers:
-    """Activations and scratch of one batch size (training keeps every
+    """Activations and scratch of one batch size, or of any up to it in
+    inference, where a pass uses the front of each (training keeps every
     layer's input for the backward pass; inference ping-pongs two).
 
     Layouts (b member, n bin, c channel, k mode, ri real/imaginary):
@@ -118,11 +119,11 @@ class _Buffers:
         self.Z16 = torch.empty(m, B, 2 * w, **bf)
         self.Zp16 = torch.empty(B * w, 2 * m, **bf)
         self.A1_16 = torch.empty(R, w, **bf)
-        self.out = torch.empty(R, net.nout, **f32)
         self.train = train
         self.lock = threading.Lock()  # held while a pass's launches go out
         if not train:
             return
+        self.out = torch.empty(R, net.nout, **f32)
         self.Vg16 = [torch.empty(w, R, **bf) for _ in range(L + 1)]
         self.Ut16 = [torch.empty(m, 2 * w, B, **bf) for _ in range(L)]
         self.Hfull = [torch.empty(R, w, **f32) for _ in range(L - 1)]
@@ -251,12 +252,15 @@ class FNO:
         return n
 
     def _buf(self, B, train):
-        """The buffers of a batch of B members.  Inference has a set per stream: passes on two
-        streams run beside each other (a training pass writes the network's gradient, so two
-        of them are not for running at a time anyway)."""
-        key = (B, True) if train else (B, False, _stream().value)
+        """Buffers for a batch of B members.  Inference has sets per stream, so that passes on
+        two streams run beside each other, each for the next power of two of members (above
+        4096 the next multiple of it), so that any number of different batch sizes keeps a few
+        sets (they stay: a captured pass may use them).  A training pass writes the network's
+        gradient, so two of them are not for running at a time anyway: one set per batch size."""
+        size = B if train else 1 << (B - 1).bit_length() if B <= 4096 else -(-B // 4096) * 4096
+        key = (B, True) if train else (size, False, _stream().value)
         if key not in self._bufs:
-            self._bufs.setdefault(key, _Buffers(self, B, train))
+            self._bufs.setdefault(key, _Buffers(self, size, train))
         return self._bufs[key]
 
     # ---- forward ----
