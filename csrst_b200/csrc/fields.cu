@@ -1215,7 +1215,10 @@ __global__ void __cluster_dims__(kFixCtas, 1, 1) __launch_bounds__(kFixThreads)
 // cell kinds in shared memory: its phases pay no L2 round trip and no cluster
 // barrier (a 46 x 28 window in FP64: 11.3 us in a step's graph), but one SM does
 // all of it, so larger windows take the cluster (a 117 x 57 window in FP32: 67
-// us in one CTA, 28 on eight).
+// us in one CTA, 28 on eight).  The line between, by a step of 4000 TSC particles,
+// us in one CTA / on the cluster: 884 cells 49.9 / 53.2 in FP64 and 43.7 / 46.3 in
+// FP32, 1872: 58.7 / 59.2 and 48.7 / 50.5, 2320: 59.4 / 58.2 and 49.7 / 50.4, 2992:
+// 64.3 / 59.5 and 51.9 / 50.7, 5568 in FP32: 66.4 / 54.2.
 template <class T>
 __host__ __device__ inline size_t fix_smem_bytes(int L0, int L1) {
   const size_t z = (size_t)(L0 + 6) * (L1 + 7), w = (size_t)(L0 + 2) * (L1 + 2);
@@ -1303,8 +1306,10 @@ struct YeeBatchFix {
   YeeFixArgs<T> x;
 };
 
-// One CTA per member: 1024 threads on its window, where the queue's 256-thread
-// CTAs took longer for one fix-up than for all of a member's tiles.
+// One CTA per member, whatever its window: 1024 threads on it, where the queue's
+// 256-thread CTAs took longer for one fix-up than for all of a member's tiles.  (With
+// many members the launch fills the chip; a batch of a few members with windows
+// beyond kFixCtaCells would do better with a cluster each.)
 template <class T>
 __global__ void __launch_bounds__(kFixThreads, 1) k_yee_fixup_batch(const YeeBatchFix<T> *fix, size_t smem_bytes) {
   yee_fixup_cta(fix[blockIdx.x].a, fix[blockIdx.x].x, smem_bytes);

@@ -5,8 +5,8 @@
 // A forward pass is 22 launches and a training step about 90, of 3 to 30 us each at
 // small batches, so a host that takes longer than that per launch is what
 // bounds them: from Python, at 23 us a launch (argument structures, views,
-// foreign calls), the wake of 37 bunches took 494 us and a 64-member training
-// step 1754 us, where the same launches replayed as a graph took 141 and 972 us.  From
+// foreign calls), the wake of 37 bunches took 426 us and a 64-member training
+// step 1677 us, where the same launches replayed as a graph took 141 and 972 us.  From
 // here a launch costs its tensor maps and the launch itself: 163 and 1155 us with
 // the kernels as they were then.  Nothing is kept between calls: every pointer comes in with the call.
 #include <cuda_runtime.h>

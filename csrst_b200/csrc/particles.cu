@@ -237,10 +237,10 @@ __device__ __forceinline__ void push_body(const PushArgs &a, const Work &work, P
 
 // The single-member push: warp tiles in dynamic shared memory, the window
 // accumulator in global memory.  It is bound by the latency of dependent FP64
-// chains (divisions and square roots among them) and, with 1640 instructions
-// per particle, by the instruction cache: the component is a template
-// parameter, the crossing list a call, the reciprocals kernel parameters, and
-// the next particle is read a round ahead.  Two CTAs per SM: at three, 80
+// chains (divisions and square roots among them); the instruction cache bound it
+// too while a particle took 1640 instructions in one kernel.  So the component is a
+// template parameter, the crossing list a call, the reciprocals kernel parameters,
+// and the next particle is read a round ahead.  Two CTAs per SM: at three, 80
 // registers a thread spill 360 bytes (8192 x 1024 mesh, 4e6 TSC particles, per
 // step: 795 us at three without the read ahead, 813 with it, 758 at two; 975
 // before).  A CTA copy of the accumulator in shared memory cost more to zero and
