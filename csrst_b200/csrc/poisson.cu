@@ -34,7 +34,7 @@
 // So a level is four line launches, and the levels of at most kTailColumns
 // columns, whose solves are latency, run as one launch of one CTA.
 //
-// 2048 x 512 mesh, 2e5 particles (8 V-cycles, with the bunch's upload): 7.7 ms,
+// 2048 x 512 mesh, 2e5 particles (8 V-cycles, with the bunch's upload): 7.4 ms,
 // 37.3 with a solver that solved each line by cyclic reduction in a CTA (9.7 - 38
 // us a launch, two divisions per row and pass), kept residual, restriction and
 // prolongation passes, and allocated its 120 arrays one by one.  A line is 4 - 8
